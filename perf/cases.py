@@ -27,7 +27,7 @@ TELESCOPE = dict(focal_length=10.7, aperture_radius=5.35, fov_deg=6.5, pixel_fov
                  paxels_on_diagonal=9, housing_overhead=1.1, reflectivity=0.9)
 DISC = dict(disc_radius=5.55, height=21.4, max_zenith_deg=1.5)
 FOUR = ("sensor", "x", "y", "time")
-HISTORY_BYTES = 72
+HISTORY_BYTES = 64
 DRAWS = 1000        # key of the draws that decide how many photons or pulses come out
 NET_FLOPS = 2.0 * (128 * 256 + 3 * 256 * 256 + 256 * 73)
 NET_PARAMS = 128 * 256 + 256 + 3 * (256 * 256 + 256) + 256 * 73 + 73
