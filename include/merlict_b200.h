@@ -248,11 +248,13 @@ typedef struct mlgpu_settings {
                                least 32.                                     */
 } mlgpu_settings;
 
-/* walk: LEVELS runs one kernel per BVH level over queued (ray, node) pairs
- * and one over the hit leaf ranges; STACK walks each ray's whole BVH in one
- * thread with a stack.  Both test the same boxes and bounding spheres and
- * find the same candidate leaves, so the results are the same.  DEFAULT is
- * LEVELS.                                                                  */
+/* walk: STACK finds each ray's closest hit in one kernel, a depth-first walk
+ * of a BVH over the leaves' surfaces; LEVELS runs one kernel per level of a
+ * BVH over their bounding spheres, over queued (ray, node) pairs, and one
+ * over the candidate leaves.  Both put every candidate through merlict's own
+ * tests, so the results are the same.  DEFAULT is STACK, and LEVELS when
+ * queue_capacity is set (the queues are the level kernels'); the pure FP32
+ * form always takes LEVELS.                                               */
 enum { MLGPU_WALK_DEFAULT = 0, MLGPU_WALK_LEVELS = 1, MLGPU_WALK_STACK = 2 };
 
 /* photon_order: COHERENT sorts the batch by a 4-D cell key of support and

@@ -410,6 +410,14 @@ int build_device_scene(mlgpu_scene* s, const mlgpu_flat_scene* f) {
             if ((st = upload(s, leaf_slot.data(), leaf_slot.size(), &s->dev.leaf_slot))) return st;
             s->dev.num_slots = (int32_t)slots;
         }
+        {
+            // the closest-hit walk's own tree over the leaves' surfaces
+            SurfBvhHost surf;
+            build_surface_bvh(f, &surf);
+            if ((st = upload(s, surf.nodes.data(), surf.nodes.size(), &s->dev.surf))) return st;
+            if ((st = upload(s, surf.leaf_ids.data(), surf.leaf_ids.size(), &s->dev.surf_leaf))) return st;
+            s->dev.surf_levels = surf.levels;
+        }
         // a tree deeper than the walk's level queues: merlict's frame walk
         if (s->dev.bvh_levels >= kMaxBvhLevels) {
             s->dev.bvh_nodes = 0;
@@ -509,14 +517,28 @@ TraceArgs make_args(const mlgpu_scene* scene, const mlgpu_photons* ph, uint64_t 
 
 constexpr uint32_t kWavePool = 1u << 21;   // ray slots of the wavefront tracers
 
+// How the rays of a call find their hits.  One thread per ray through the
+// surface BVH (STACK) unless the caller asks for the level kernels, by name
+// or by the size of their queues; the pure FP32 form always takes them: its
+// textbook roots can lie further outside a surface than that BVH's boxes.
+int wave_walk(const mlgpu_scene* scene, const mlgpu_settings* st) {
+    if (st->tracer == MLGPU_TRACER_FP32_PURE || st->walk == MLGPU_WALK_LEVELS ||
+        (st->walk == MLGPU_WALK_DEFAULT && st->queue_capacity != 0) ||
+        (scene->dev.surf_levels == 0 && scene->dev.bvh_nodes > 0))
+        return MLGPU_WALK_LEVELS;
+    return MLGPU_WALK_STACK;
+}
+
 // Carves the two ray pools, the candidate lists and the counters out of
 // one device buffer.
 int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32_t queue_cap,
-                 WaveBuffers* w, RayPool* p0, RayPool* p1) {
+                 int walk, WaveBuffers* w, RayPool* p0, RayPool* p1) {
     auto up = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t P = pool;
-    const size_t level_cap = queue_cap ? queue_cap : 8*P;
-    const size_t isect_cap = queue_cap ? queue_cap : 16*P;
+    // the queues are the level kernels'
+    const bool queues = walk == MLGPU_WALK_LEVELS;
+    const size_t level_cap = !queues ? 0 : queue_cap ? queue_cap : 8*P;
+    const size_t isect_cap = !queues ? 0 : queue_cap ? queue_cap : 16*P;
     const size_t per_pool = up(P*48) + 3*up(P*8) + 8*up(P*4) + 2*up(P*16);
     const size_t rest = 2*up(level_cap*8) + up(isect_cap*8) + up(isect_cap*8) + up(P*4);
     MLGPU_CUDA(scene->wave.reserve(kWaveCounterBytes + 2*per_pool + rest));
@@ -665,10 +687,11 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     const uint32_t pool = (uint32_t)std::min<uint64_t>(a.num_photons, want);
     WaveBuffers w;
     RayPool pools[2];
+    const int walk = wave_walk(scene, st);
     const int rc = wave_buffers(scene, pool, st->grid_blocks, st->staged_levels,
-                                st->queue_capacity, &w, &pools[0], &pools[1]);
+                                st->queue_capacity, walk, &w, &pools[0], &pools[1]);
     if (rc) return rc;
-    w.walk = st->walk == MLGPU_WALK_STACK ? MLGPU_WALK_STACK : MLGPU_WALK_LEVELS;
+    w.walk = walk;
     // per-kernel events cannot be taken inside a graph: profiling runs launch by launch
     const bool graph = st->use_graph != 0 && !scene->prof.on;
     int period = st->check_period > 0 ? st->check_period : 4;
@@ -708,13 +731,15 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
         a.max_interactions + 16 + (uint64_t)period*(feed ? feed->pieces + 1 : 1);
     // launches per iteration: intake and its counters, the walk, intersections
     // and ties, the overflow walk, resolve and its counters
-    const int walk_launches = w.walk == MLGPU_WALK_STACK ? 1 : scene->dev.bvh_levels;
+    const bool stack = w.walk == MLGPU_WALK_STACK;
+    const int walk_launches = stack ? 1 : scene->dev.bvh_levels;
+    const int iteration_launches = stack ? 5 : walk_launches + 7;
     uint64_t iteration = 0;
     while (true) {
         if (graph) {
             MLGPU_CUDA(cudaGraphLaunch(scene->wave_graph, stream));
             iteration += (uint64_t)period;
-            scene->launches += (uint64_t)period*((uint64_t)walk_launches + 7) + 1;
+            scene->launches += (uint64_t)period*(uint64_t)iteration_launches + 1;
         } else {
             for (int g = 0; g < period; g++, iteration++) {
                 const RayPool& cur = pools[iteration & 1];
@@ -724,12 +749,13 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
                 const cudaError_t e = launch_wave_iteration(a, w, cur, nxt, form, stream,
                                                             timed ? ch.ev : nullptr);
                 if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
-                scene->launches += (uint64_t)walk_launches + 7;
+                scene->launches += (uint64_t)iteration_launches;
                 if (timed) {
                     ch.n = 5;
                     const int cls[4] = {MLGPU_KERNEL_INTAKE, MLGPU_KERNEL_WALK,
                                         MLGPU_KERNEL_INTERSECT, MLGPU_KERNEL_RESOLVE};
-                    const int launches[4] = {2, walk_launches, 2, 3};
+                    const int launches[4] = {stack ? 0 : 2, stack ? 3 : walk_launches,
+                                             stack ? 0 : 2, stack ? 2 : 3};
                     for (int k = 0; k < 4; k++) { ch.cls[k] = cls[k]; ch.launches[k] = launches[k]; }
                     scene->prof.add(ch);
                 }
@@ -751,7 +777,7 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
             }
             // an empty pool with the next piece still on its way: the trace
             // stream waits for that piece (no kernel spins on it)
-            if (h.active == 0 && h.next_input == h.avail_snap && h.next_input < a.num_photons) {
+            if (h.active + h.inside == 0 && h.next_input == h.avail_snap && h.next_input < a.num_photons) {
                 int c = 0;
                 while (c + 1 < feed->pieces && feed->start[c + 1] <= h.next_input) c++;
                 MLGPU_CUDA(cudaStreamWaitEvent(stream, feed->ord_ready[c], 0));
@@ -759,7 +785,7 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
                 scene->launches++;
             }
         }
-        if (h.active == 0 && h.next_input >= a.num_photons) break;
+        if (h.active + h.inside == 0 && h.next_input >= a.num_photons) break;
         if (iteration > bound)
             return fail(MLGPU_ERR_RUNTIME, "wavefront tracer did not drain its pool");
     }

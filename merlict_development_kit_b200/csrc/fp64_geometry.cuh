@@ -41,6 +41,14 @@ __device__ __forceinline__ v3 divide(v3 a, double s) { return mk(a.x/s, a.y/s, a
 __device__ __forceinline__ double norm(v3 a) { return sqrt(a.x*a.x + a.y*a.y + a.z*a.z); }
 __device__ __forceinline__ v3 normalized(v3 a) { return divide(a, norm(a)); }
 
+// The same without contraction whatever the translation unit's --fmad: a
+// photon's direction is merlict's in the single-precision forms too.
+__device__ __forceinline__ v3 normalized_rn(v3 a) {
+    const double n = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)),
+                                          __dmul_rn(a.z, a.z)));
+    return mk(__ddiv_rn(a.x, n), __ddiv_rn(a.y, n), __ddiv_rn(a.z, n));
+}
+
 // HomTra3 (merlict/HomTra3.cpp:154-216); T holds the three rows.
 __device__ __forceinline__ v3 orientation(const double* t, v3 v) {
     return mk(v.x*t[0] + v.y*t[1] + v.z*t[2],
@@ -195,7 +203,7 @@ __device__ __forceinline__ void set_isec(Isec* r, int32_t leaf, v3 p, v3 n, doub
 }
 
 // SurfaceWithOuterPrismBound::add_causeal_intersection, SurfaceWithOuterPrismBound.cpp:7-70
-__device__ void add_causal(const DevScene& sc, int32_t leaf, int32_t prim, const double* pr,
+__device__ __forceinline__ void add_causal(const DevScene& sc, int32_t leaf, int32_t prim, const double* pr,
                            double r2, double plus, double minus, v3 s, v3 d, Isec* out) {
     const v3 pi = add(s, scale(d, plus));
     const v3 mi = add(s, scale(d, minus));
@@ -225,9 +233,10 @@ __device__ __forceinline__ double tri_sign(v3 p1, double p2x, double p2y, double
 }
 
 // calculate_intersection_with of the leaf primitives
-// (merlict/scenery/primitive), ray given in the leaf's frame.
-__device__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
-                               const double* pr, double r2, v3 s, v3 d, Isec* out) {
+// (merlict/scenery/primitive), ray given in the leaf's frame, in three
+// classes of arithmetic (leaf_class).
+__device__ __forceinline__ void intersect_cap(const DevScene& sc, int32_t leaf, int32_t prim,
+                                              const double* pr, double r2, v3 s, v3 d, Isec* out) {
     out->leaf = -1;
     switch (prim) {
     case MLGPU_PRIM_SPHERE_CAP_HEX:
@@ -253,6 +262,15 @@ __device__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
             add_causal(sc, leaf, prim, pr, r2, plus, minus, s, d, out);
         break;
     }
+    default:
+        break;
+    }
+}
+
+__device__ __forceinline__ void intersect_plane(const DevScene& sc, int32_t leaf, int32_t prim,
+                                                const double* pr, v3 s, v3 d, Isec* out) {
+    out->leaf = -1;
+    switch (prim) {
     case MLGPU_PRIM_DISC:
     case MLGPU_PRIM_HEX_PLANE:
     case MLGPU_PRIM_PLANE:
@@ -291,6 +309,15 @@ __device__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
         if (inside && differs(s, p)) set_isec(out, leaf, p, mk(0.0, 0.0, 1.0), v, d);
         break;
     }
+    default:
+        break;
+    }
+}
+
+__device__ __forceinline__ void intersect_quadric(int32_t leaf, int32_t prim, const double* pr,
+                                                  v3 s, v3 d, Isec* out) {
+    out->leaf = -1;
+    switch (prim) {
     case MLGPU_PRIM_CYLINDER: {
         // ZaxisCylinderRayIntersectionEquation.cpp:6-86, Cylinder.cpp:121-150
         const double radius = pr[0], length = pr[1];
@@ -332,6 +359,15 @@ __device__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
     }
     default:
         break;
+    }
+}
+
+__device__ __forceinline__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
+                                               const double* pr, double r2, v3 s, v3 d, Isec* out) {
+    switch (leaf_class(prim)) {
+    case kLeafCap: intersect_cap(sc, leaf, prim, pr, r2, s, d, out); break;
+    case kLeafPlane: intersect_plane(sc, leaf, prim, pr, s, d, out); break;
+    default: intersect_quadric(leaf, prim, pr, s, d, out); break;
     }
 }
 
@@ -381,14 +417,14 @@ __device__ __forceinline__ void test_candidate(const DevScene& sc, int32_t leaf,
 }
 
 // merlict's intersection of one leaf with a world ray; leaf < 0 if none.
-// The leaf record in 16-byte loads: the first line (transform, inverse
-// translation, primitive), the squared radius with the first parameter, and
-// only as many further parameter pairs as the primitive has parameters --
-// a warp whose lanes hold different leaves issues one request per lane and
-// load, so every load left out counts.
+// The leaf record in 32-byte loads: transform, inverse translation,
+// primitive, squared radius and three parameters, and the other parameters
+// only where the primitive has them -- a warp whose lanes hold different
+// leaves takes one pass of the L1 per lane and load, however wide the load,
+// so every load left out counts.
 static_assert(offsetof(LeafRec, tinv) == 96 && offsetof(LeafRec, primitive) == 120 &&
               offsetof(LeafRec, r2) == 128 && offsetof(LeafRec, params) == 136,
-              "load_leaf reads the leaf record in 16-byte pieces");
+              "load_leaf reads the leaf record in 32-byte pieces");
 __device__ __forceinline__ int primitive_params(int32_t prim) {
     switch (prim) {
     case MLGPU_PRIM_DISC: case MLGPU_PRIM_HEX_PLANE: case MLGPU_PRIM_SPHERE: return 1;
@@ -402,30 +438,29 @@ __device__ __forceinline__ int primitive_params(int32_t prim) {
     }
 }
 
+__device__ __forceinline__ void load4(const double* p, double* v) {
+    asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+        : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
 __device__ __forceinline__ void load_leaf(const LeafRec* L, double* T, double* ti, double* pr,
                                           double* r2, int32_t* prim) {
-    const double2* q = reinterpret_cast<const double2*>(L);
-    double v[14];
+    const double* q = reinterpret_cast<const double*>(L);
+    double v[20];
 #pragma unroll
-    for (int k = 0; k < 7; k++) {
-        const double2 x = __ldg(q + k);
-        v[2*k] = x.x;
-        v[2*k + 1] = x.y;
-    }
-    const double2 tail = __ldg(q + 7);                     // tinv[2], primitive | sensor
-    const double2 r2p0 = __ldg(q + 8);                     // r2, params[0]
+    for (int k = 0; k < 5; k++) load4(q + 4*k, v + 4*k);   // to params[2]
 #pragma unroll
     for (int k = 0; k < 12; k++) T[k] = v[k];
-    ti[0] = v[12]; ti[1] = v[13]; ti[2] = tail.x;
-    *prim = (int32_t)(uint32_t)(__double_as_longlong(tail.y) & 0xffffffffll);
-    *r2 = r2p0.x;
-    pr[0] = r2p0.y;
+    ti[0] = v[12]; ti[1] = v[13]; ti[2] = v[14];
+    *prim = (int32_t)(uint32_t)(__double_as_longlong(v[15]) & 0xffffffffll);
+    *r2 = v[16];
+    pr[0] = v[17]; pr[1] = v[18]; pr[2] = v[19];
 #pragma unroll
-    for (int k = 1; k < MLGPU_LEAF_PARAMS; k++) pr[k] = 0.0;
-    const int np = primitive_params(*prim);
-    if (np > 1) { const double2 x = __ldg(q + 9); pr[1] = x.x; pr[2] = x.y; }
-    if (np > 3) { const double2 x = __ldg(q + 10); pr[3] = x.x; pr[4] = x.y; }
-    if (np > 5) { const double2 x = __ldg(q + 11); pr[5] = x.x; pr[6] = x.y; }
+    for (int k = 3; k < MLGPU_LEAF_PARAMS; k++) pr[k] = 0.0;
+    if (primitive_params(*prim) > 3) {
+        load4(q + 20, v);
+        pr[3] = v[0]; pr[4] = v[1]; pr[5] = v[2]; pr[6] = v[3];
+    }
 }
 
 // load_leaf on the slot-ordered candidate records (DevScene::slot_rec):
@@ -457,14 +492,27 @@ __device__ __forceinline__ void load_leaf_slot(const DevScene& sc, uint32_t j, d
     if (np > 5) { const double2 x = __ldg(q + 8*11); pr[5] = x.x; pr[6] = x.y; }
 }
 
-__device__ __forceinline__ Isec leaf_hit(const DevScene& sc, int32_t leaf, v3 s, v3 d) {
-    double T[12], ti[3], pr[MLGPU_LEAF_PARAMS], r2;
+// The intersection of leaf `leaf` at the distance that intersect_leaf found:
+// the same point and normal, without solving for the distance again.  `T`
+// receives the leaf's transform.
+__device__ __forceinline__ void hit_at(const DevScene& sc, int32_t leaf, double dist, v3 s, v3 d,
+                                       double* T, Isec* out) {
+    double ti[3], pr[MLGPU_LEAF_PARAMS], r2;
     int32_t prim;
     load_leaf(sc.leaf + leaf, T, ti, pr, &r2, &prim);
-    Isec h;
-    intersect_leaf(sc, leaf, prim, pr, r2, position_inverse(T, ti, s), orientation_inverse(T, d),
-                   &h);
-    return h;
+    const v3 ls = position_inverse(T, ti, s), ld = orientation_inverse(T, d);
+    const v3 p = add(ls, scale(ld, dist));
+    v3 n = mk(0.0, 0.0, 1.0);
+    switch (leaf_class(prim)) {
+    case kLeafCap: n = cap_normal(prim, pr, p); break;
+    case kLeafPlane: break;
+    default: {
+        const v3 q = prim == MLGPU_PRIM_CYLINDER ? mk(p.x, p.y, 0.0) : p;
+        n = divide(q, norm(q));
+        break;
+    }
+    }
+    set_isec(out, leaf, p, n, dist, ld);
 }
 
 constexpr int kCandidates = 16;

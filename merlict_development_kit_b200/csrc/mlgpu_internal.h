@@ -101,6 +101,43 @@ struct __align__(16) QNode {
 static_assert(sizeof(QNode) == 96 && kBvhWidth == 8, "QNode: six 16-byte words, eight children");
 void quantise_bvh_node(const BvhNode& n, QNode* q);
 
+// A node of the surface BVH (closest_hit.cuh): eight child slots whose boxes
+// bound the leaves' surfaces (not their bounding spheres), 96 bytes read as
+// three 32-byte words: origin, the three biased exponents in bytes 0-2 and
+// the mask of slots that are nodes in byte 3, the node of slot 0, first leaf
+// slot << 8 | mask of slots that are single leaves, and their classes; then
+// the bounds as in QNode.  The node in slot k is child_base + k; the leaves
+// of a node sit one after another from its first leaf slot, in slot order.
+// Slots are given to children by octant: bit a of a slot is set when the
+// child lies towards the high side of axis a, so that visiting slots in the
+// order of (slot ^ octant of the ray's direction) runs front to back.
+struct __align__(32) SurfNode {
+    float origin[3];
+    uint32_t exps_nodes;
+    uint32_t child_base;
+    uint32_t leaf_base_mask;
+    uint32_t leaf_kinds;    // slots that are caps, planes, leaves (a byte each)
+    uint32_t pad;
+    uint32_t qlo[3][2];
+    uint32_t qhi[3][2];
+    uint32_t pad2[4];
+};
+static_assert(sizeof(SurfNode) == 96, "SurfNode: three 32-byte words");
+// The leaves' classes of arithmetic: what a warp intersects together.
+enum { kLeafCap = 0, kLeafPlane = 1, kLeafQuadric = 2 };
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int leaf_class(int32_t primitive) {
+    switch (primitive) {
+    case MLGPU_PRIM_SPHERE_CAP_HEX: case MLGPU_PRIM_SPHERE_CAP_CYL:
+    case MLGPU_PRIM_SPHERE_CAP_RECT: case MLGPU_PRIM_ELLIPTIC_CAP_HEX: return kLeafCap;
+    case MLGPU_PRIM_CYLINDER: case MLGPU_PRIM_SPHERE: case MLGPU_PRIM_NONE: return kLeafQuadric;
+    default: return kLeafPlane;
+    }
+}
+constexpr int kMaxSurfLevels = 64;      // the walk's stack holds one entry per level
+
 constexpr int32_t kBvhLeafFlag = (int32_t)0x80000000u;
 constexpr int32_t kBvhEmpty = 0x7fffffff;
 constexpr int kBvhStack = 64;
@@ -124,6 +161,10 @@ struct DevScene {
     double hex_u[3], hex_v[3], hex_w[3];
     unsigned int* error_word;   // first device-side error code
     // BVH over the leaves with geometry (empty: walk the frame tree)
+    // the surface BVH of the closest-hit walk (surf_levels = 0: none)
+    const SurfNode* surf;
+    const int32_t* surf_leaf;   // [leaves with geometry] leaf of each leaf slot
+    int32_t surf_levels;
     const BvhNode* bvh;
     const QNode* bvh_q;         // the same nodes quantised (the level kernels read these)
     const int32_t* bvh_leaf;
@@ -209,12 +250,23 @@ struct BvhHost {
 };
 void build_bvh(const mlgpu_flat_scene* f, double inflate, BvhHost* out);
 
+// The surface BVH (bvh_build.cu).  levels == 0: the tree does not fit the
+// node's fields or the walk's stack.
+struct SurfBvhHost {
+    std::vector<SurfNode> nodes;        // the root first; unused slots of a parent are zero
+    std::vector<int32_t> leaf_ids;      // leaf of each leaf slot
+    int levels = 0;
+};
+void build_surface_bvh(const mlgpu_flat_scene* f, SurfBvhHost* out);
+
 // wavefront tracers: a pool of ray slots, two of them (current, next)
 struct WaveCounters {
     unsigned long long next_input;   // photons taken into the pool so far
-    unsigned int active;             // rays carried over into the current pool
+    unsigned int active;             // rays carried over into the current pool, from its start
+    unsigned int inside;             // and from its end: rays inside a lens (closest-hit walk)
     unsigned int total;              // active + new photons of this iteration
     unsigned int next;               // survivors written to the next pool
+    unsigned int next_inside;        // of them, from its end
     unsigned int isect_len;          // (slot, leaf) candidates to intersect
     unsigned int overflow_len;       // slots sent to merlict's own walk
     unsigned int level_len[kMaxBvhLevels];   // (slot, node) pairs of each BVH level
@@ -280,6 +332,12 @@ cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* ho
                                          cudaStream_t s);
 // the FP32 forms' intersection and resolve kernels; `mid` (may be null) is
 // recorded between them
+void launch_wave32_hit(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                       cudaStream_t s);
+void launch_wave32_tree(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur, int front,
+                        cudaStream_t s);
+void launch_wave32_resolve(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                           const RayPool& nxt, bool pure, cudaStream_t s);
 cudaError_t launch_wave32_isect_resolve(const TraceArgs& a, const WaveBuffers& w,
                                         const RayPool& cur, const RayPool& nxt, bool pure,
                                         cudaStream_t s, cudaEvent_t mid);

@@ -26,8 +26,7 @@
 #include <climits>
 #include <cstdint>
 
-#include "fp64_geometry.cuh"
-#include "fp32_geometry.cuh"
+#include "closest_hit.cuh"
 #include "merlict_b200_philox.h"
 
 namespace mlgpu {
@@ -35,17 +34,10 @@ namespace {
 
 using namespace fp64;
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kNoStep = -2;             // step state: the photon takes no step
 constexpr int kStepNone = 0;            // it takes a step; nothing to queue (no candidates)
 constexpr int kStepBvh = 1;             // it takes a step; the intake queues the BVH root
 constexpr int kStepTree = 2;            // it takes a step; the intake walks its frame subtree
-constexpr int32_t kNoLeaf = INT32_MAX;  // best_leaf of a ray without a hit
-constexpr unsigned long long kNoKey = ~0ull;
-
-constexpr int kIsectFp64 = 0;
-constexpr int kIsectFp32 = 1;
-constexpr int kIsectFp32Pure = 2;
 
 template <typename T>
 __device__ __forceinline__ double load_in(const void* p, uint64_t i) {
@@ -112,19 +104,31 @@ __device__ __forceinline__ float box_inflation(const DevScene& sc, float ox, flo
     return sc.bvh_eps + 4e-7f*(fabsf(ox) + fabsf(oy) + fabsf(oz));
 }
 
-// What the next intake queues for a ray about to take a step from s along d
-// in the frame subtree `root`, and its FP32 walk record when that is the
-// BVH: inside a lens (root != 0), or without a BVH, merlict's own walk of
-// the subtree (kStepTree); else merlict tests the root frame's sphere first
-// (RayAndFrame.cpp:137-149) and the BVH walk follows if the ray passes it.
-__device__ __forceinline__ int prepare_walk(const TraceArgs& a, const RayPool& p, uint32_t slot,
-                                            v3 s, v3 d, int32_t root) {
+// How a ray about to take a step from s along d in the frame subtree `root`
+// finds its hit: inside a lens (root != 0), or without a BVH, by merlict's
+// own walk of the subtree (kStepTree); else merlict tests the root frame's
+// sphere first (RayAndFrame.cpp:137-149) and the BVH walk follows if the ray
+// passes it.
+__device__ __forceinline__ int step_kind(const TraceArgs& a, const WaveBuffers& w, v3 s, v3 d,
+                                         int32_t root) {
     const DevScene& sc = a.scene;
-    if (root != 0 || sc.bvh_nodes == 0 || a.traversal == MLGPU_TRAVERSAL_FRAME_TREE)
+    if (root != 0 || (w.walk == MLGPU_WALK_LEVELS ? sc.bvh_nodes : sc.surf_levels) == 0 ||
+        a.traversal == MLGPU_TRAVERSAL_FRAME_TREE)
         return kStepTree;
     const double2* np = reinterpret_cast<const double2*>(sc.node);
     const double2 n01 = __ldg(np), n23 = __ldg(np + 1);
-    if (!sphere_cull(make_double4(n01.x, n01.y, n23.x, n23.y), s, d, dot(s, d))) return kStepNone;
+    return sphere_cull(make_double4(n01.x, n01.y, n23.x, n23.y), s, d, dot(s, d)) ? kStepBvh
+                                                                                 : kStepNone;
+}
+
+// What the level kernels keep of a ray in slot `slot`: its cleared closest
+// hit and, for a BVH walk, its FP32 walk record.
+__device__ __forceinline__ void prepare_levels(const DevScene& sc, const RayPool& p, uint32_t slot,
+                                               v3 s, v3 d, int step) {
+    p.best_key[slot] = kNoKey;
+    p.best_leaf[slot] = kNoLeaf;
+    p.overflow_flag[slot] = 0u;
+    if (step != kStepBvh) return;
     const float ox = (float)s.x, oy = (float)s.y, oz = (float)s.z;
     float fdx = (float)d.x, fdy = (float)d.y, fdz = (float)d.z;
     if (fabsf(fdx) < 1e-30f) fdx = copysignf(1e-30f, fdx);
@@ -132,7 +136,164 @@ __device__ __forceinline__ int prepare_walk(const TraceArgs& a, const RayPool& p
     if (fabsf(fdz) < 1e-30f) fdz = copysignf(1e-30f, fdz);
     p.ray_o[slot] = make_float4(ox, oy, oz, box_inflation(sc, ox, oy, oz));
     p.ray_i[slot] = make_float4(1.0f/fdx, 1.0f/fdy, 1.0f/fdz, 0.0f);
-    return kStepBvh;
+}
+
+// A new photon into slot `slot`: the next of the batch's tracing order
+// (merlict::Photon's constructor, Ray.cpp:16-20, RayForPropagation.cpp:52-64),
+// prepared like the survivors the previous resolve step prepared.  Returns
+// its step.
+template <typename In>
+__device__ __forceinline__ int admit_photon(const TraceArgs& a, const WaveBuffers& w,
+                                            const RayPool& cur, uint32_t slot, uint64_t q,
+                                            v3* support, v3* direction) {
+    const uint32_t max_int = a.max_interactions;
+    uint64_t p;
+    v3 s, d;
+    double lambda;
+    if (a.sorted) {
+        // the photon's record in tracing order
+        const double2* r = a.sorted + 4*q;
+        const double2 r0 = __ldcg(r), r1 = __ldcg(r + 1), r2 = __ldcg(r + 2), r3 = __ldcg(r + 3);
+        s = mk(r0.x, r0.y, r1.x);
+        d = normalized_rn(mk(r1.y, r2.x, r2.y));
+        lambda = r3.x;
+        p = (uint64_t)__double_as_longlong(r3.y);
+    } else {
+        p = a.order ? (uint64_t)__ldg(a.order + q) : q;
+        s = mk(load_in<In>(a.photons.sx, p), load_in<In>(a.photons.sy, p),
+               load_in<In>(a.photons.sz, p));
+        d = normalized_rn(mk(load_in<In>(a.photons.dx, p), load_in<In>(a.photons.dy, p),
+                          load_in<In>(a.photons.dz, p)));
+        lambda = load_in<In>(a.photons.wavelength, p);
+    }
+    const int32_t root = a.start_node;
+    cur.photon[slot] = (int32_t)p;
+    store_ray(cur, slot, s, d);
+    // Photon::assert_wavelength_is_positive (Photon.cpp:20-28): merlict
+    // throws std::invalid_argument before propagating
+    if (lambda <= 0.0) raise_error(a.scene.error_word, MLGPU_ERR_INVALID_ARGUMENT);
+    cur.lambda[slot] = lambda;
+    cur.tof[slot] = 0.0;
+    cur.root[slot] = root;
+    cur.n_int[slot] = 1;
+    cur.k_draw[slot] = 0;
+    cur.err[slot] = 0;
+    if (a.results.history)
+        store_hist(a.results.history + p*(max_int + 1), s, d, 0.0, MLGPU_LEAF_PHOTON_SOURCE,
+                   MLGPU_PRODUCTION, dot(d, d) < 0.0);
+    const int step = 1u > max_int ? kNoStep : step_kind(a, w, s, d, root);
+    if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(a.scene, cur, slot, s, d, step);
+    cur.step[slot] = step;
+    *support = s;
+    *direction = d;
+    return step;
+}
+
+// Intake and closest hit in one kernel: new photons enter the free slots,
+// and every ray that takes a step finds its closest hit (closest_hit.cuh)
+// for the resolve step.  The grid's warps take the pool's slots in chunks of
+// 32; a lane whose ray has been walked takes the next slot once kRefill
+// lanes are free, so that a warp's lanes stay busy although rays visit
+// different numbers of nodes.
+constexpr int kRefill = 16;
+
+template <typename In, int kIsect>
+__global__ void __launch_bounds__(kWalkThreads, kWalkBlocks)
+wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
+    extern __shared__ double2 s_walk[];
+    const DevScene& sc = a.scene;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kWalkThreads/32;
+    WalkWarp* sw = reinterpret_cast<WalkWarp*>(s_walk) + warp;
+    uint32_t* stack = reinterpret_cast<uint32_t*>(reinterpret_cast<WalkWarp*>(s_walk) + kWarps) +
+        threadIdx.x;
+    const uint32_t active = w.counters->active;
+    const unsigned long long next_input = w.counters->next_input;
+    // a fed propagation admits only the photons whose records have arrived
+    const unsigned long long limit = a.fed ? w.counters->avail_snap : a.num_photons;
+    const unsigned long long remaining = limit - next_input;
+    const uint32_t inside = w.counters->inside;
+    const uint32_t room = w.pool - active - inside;
+    const uint32_t total = active + (uint32_t)(remaining < room ? remaining : room);
+    const uint32_t chunks = (total + 31)/32, stride = gridDim.x*kWarps;
+    uint32_t chunk = blockIdx.x*kWarps + warp;
+    int taken = 0;               // slots of this chunk given out
+    WalkLane l;
+    l.walking = false;
+    l.eps = 0.0f;
+    l.key = kNoKey;
+    uint32_t slot = 0;
+    bool have = false;           // the lane holds a ray whose hit is not written yet
+    uint32_t listed = 0;         // lengths of the lists
+    int groups = 0;
+    while (true) {
+        const unsigned idle = __ballot_sync(kFull, !l.walking);
+        const int free_lanes = __popc(idle);
+        const bool refill = free_lanes == 32 || (free_lanes >= kRefill && chunk < chunks);
+        while (groups >= 32 || (refill && (groups | (int)listed) != 0)) {
+            groups = spread_groups(sw, lane, groups, &listed);
+            listed = work_off<kIsect>(sc, sw, lane, listed, refill && groups == 0 ? 1 : 32, &l);
+        }
+        if (refill) {
+            const bool is_free = (idle >> lane) & 1u;
+            if (is_free && have) {
+                cur.best_leaf[slot] = sw->leaf[lane];
+                cur.best_key[slot] = sw->key[lane];
+                have = false;
+            }
+            if (chunk >= chunks) break;   // all lanes are free and no slots are left
+            const int rank = __popc(idle & ((1u << lane) - 1u));
+            const int take = min(free_lanes, 32 - taken);
+            const uint32_t next = chunk*32u + (uint32_t)(taken + rank);
+            if (is_free && rank < take && next < total) {
+                slot = next;
+                v3 s, d;
+                int step;
+                if (slot >= active) {
+                    step = admit_photon<In>(a, w, cur, slot, next_input + (slot - active), &s, &d);
+                } else {
+                    step = cur.step[slot];
+                    load_ray(cur, slot, &s, &d);
+                }
+                if (step == kStepBvh) {
+                    walk_begin(sc, s, d, sw, lane, &l);
+                    have = true;
+                } else {
+                    cur.best_leaf[slot] = kNoLeaf;
+                }
+            }
+            taken += take;
+            if (taken == 32) { chunk += stride; taken = 0; }
+            __syncwarp();
+        }
+        uint2 group = make_uint2(0u, 0u);
+        if (l.walking) group = walk_step(sc, &l, stack);
+        const unsigned reached = __ballot_sync(kFull, (group.x & 0xffu) != 0);
+        if ((group.x & 0xffu) != 0)
+            sw->group[groups + __popc(reached & ((1u << lane) - 1u))] =
+                make_uint2(group.x, group.y | (uint32_t)lane << 24);
+        groups += __popc(reached);
+        __syncwarp();
+    }
+}
+
+// The rays whose hit merlict's own walk of a frame subtree finds: those
+// inside a lens, from the pool's end, and with `front` also new photons
+// (start_node inside a subtree, no BVH, or the frame tree asked for).
+template <int kIsect>
+__global__ void __launch_bounds__(128)
+wave_tree_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int front) {
+    const uint32_t inside = w.counters->inside;
+    const uint32_t rays = inside + (front ? w.counters->total : 0u);
+    for (uint32_t k = blockIdx.x*blockDim.x + threadIdx.x; k < rays; k += gridDim.x*blockDim.x) {
+        const uint32_t slot = k < inside ? w.pool - 1u - k : k - inside;
+        if (cur.step[slot] != kStepTree) continue;
+        v3 s, d;
+        load_ray(cur, slot, &s, &d);
+        double dist;
+        cur.best_leaf[slot] = closest_hit_tree<kIsect>(a.scene, cur.root[slot], s, d, &dist);
+        cur.best_key[slot] = (unsigned long long)__double_as_longlong(dist);
+    }
 }
 
 template <int kIsect>
@@ -195,13 +356,17 @@ wave_overflow_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) 
         load_ray(cur, slot, &s, &d);
         const Isec is = first_intersection_tree(a.scene, cur.root[slot], s, d);
         cur.best_leaf[slot] = is.leaf >= 0 ? is.leaf : kNoLeaf;
+        cur.best_key[slot] = (unsigned long long)__double_as_longlong(is.dist);
     }
 }
 
 // Three blocks per SM (80 registers, a few hundred bytes spilled): measured
 // faster than two blocks at 126 registers.
+constexpr int kResolveThreads = 128;
+constexpr int kResolveBlocks = 7;
+
 template <typename Out, int kIsect>
-__global__ void __launch_bounds__(256, 3)
+__global__ void __launch_bounds__(kResolveThreads, kResolveBlocks)
 wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, const RayPool nxt) {
     const DevScene& sc = a.scene;
     // the property tables, staged in shared memory when they fit
@@ -218,9 +383,10 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
         fn_off = s_off;
     }
     const uint32_t total = w.counters->total;
-    const uint32_t slot = blockIdx.x*blockDim.x + threadIdx.x;
+    const uint32_t index = blockIdx.x*blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
-    const bool valid = slot < total;
+    const bool valid = index < total + w.counters->inside;
+    const uint32_t slot = index < total ? index : w.pool - 1u - (index - total);
     const uint32_t max_int = a.max_interactions;
     const uint32_t hist_len = max_int + 1;
 
@@ -252,8 +418,7 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
 
         Isec is;
         int kind = MLGPU_PRODUCTION;
-        bool moved = false;
-        v3 new_s = s, new_d = d;
+        bool moved = false;      // then s and d are the photon's new ray
         double T[12];
         if (count == kNoStep) {
             is.leaf = MLGPU_LEAF_PHOTON_SOURCE;
@@ -264,13 +429,13 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             // merlict's closest hit among the candidates: minimum distance,
             // ties to merlict's visiting order (RayAndFrame.cpp:160-173)
             {
-                // the winner of the intersection and tie kernels (or of
-                // merlict's own walk), recomputed by the same code
+                // the winner of the search at its distance; the FP32 forms
+                // intersect it again with the hit point refined
                 const int32_t best = cur.best_leaf[slot];
                 if (best == kNoLeaf) {
                     set_void(&is, s, d);
                 } else if (kIsect == kIsectFp64) {
-                    is = leaf_hit(sc, best, s, d);
+                    hit_at(sc, best, __longlong_as_double((long long)cur.best_key[slot]), s, d, T, &is);
                 } else {
                     const fp32::Hit32 h = fp32::intersect32<true>(sc, best, fp32::dmk(s.x, s.y, s.z),
                                                             fp32::dmk(d.x, d.y, d.z),
@@ -288,32 +453,17 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             }
             const bool hit = is.leaf >= 0;
             const LeafRec* L = hit ? sc.leaf + is.leaf : nullptr;
-            if (hit) {
-                const double2* q = reinterpret_cast<const double2*>(L->T);
+            if (hit && kIsect != kIsectFp64) {
 #pragma unroll
-                for (int k = 0; k < 6; k++) {
-                    const double2 x = __ldg(q + k);
-                    T[2*k] = x.x;
-                    T[2*k + 1] = x.y;
-                }
-            } else {
+                for (int k = 0; k < 3; k++) load4(L->T + 4*k, T + 4*k);
+            } else if (!hit) {
 #pragma unroll
                 for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
             }
-            int32_t fn[6] = {0, 0, 0, 0, 0, 0};
-            int32_t flags = 0, allowed = -1;
-            if (hit) {
-                static_assert(offsetof(LeafRec, allowed_node) == 200 &&
-                              offsetof(LeafRec, flags) == 204 && offsetof(LeafRec, fn) == 208,
-                              "the resolve step reads these fields in 8- and 16-byte pieces");
-                const int2 af = __ldg(reinterpret_cast<const int2*>(&L->allowed_node));
-                const int4 f03 = __ldg(reinterpret_cast<const int4*>(L->fn));
-                const int2 f45 = __ldg(reinterpret_cast<const int2*>(L->fn + 4));
-                allowed = af.x;
-                flags = af.y;
-                fn[0] = f03.x; fn[1] = f03.y; fn[2] = f03.z; fn[3] = f03.w;
-                fn[4] = f45.x; fn[5] = f45.y;
-            }
+            // a property table of the surface, by the side the ray comes from
+            auto table = [&](int outside, int inside) {
+                return __ldg(L->fn + (is.outside ? outside : inside));
+            };
             auto draw = [&]() -> double {
                 const uint32_t k = (uint32_t)k_draw++;
                 if (a.rng.mode == MLGPU_RNG_REPLAY) {
@@ -325,30 +475,32 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             bool absorbed = false;
             if (hit) {
                 // absorbed_in_medium_before_reaching_surface, PhotonAndFrame.cpp:32-38
-                const double depth = func_eval_tab(fn_pts, fn_off, fn[is.outside ? MLGPU_SURF_OUTER_ABSORPTION
-                                                                  : MLGPU_SURF_INNER_ABSORPTION], lambda, &err);
-                const double survival = exp(-is.dist/depth);
-                absorbed = draw() > survival;
+                const double depth = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_ABSORPTION, MLGPU_SURF_INNER_ABSORPTION), lambda, &err);
+                if (depth != depth && a.rng.mode == MLGPU_RNG_PHILOX) {
+                    // merlict's default table evaluates to NaN, and no draw
+                    // is larger than that: only the draw is counted
+                    k_draw++;
+                } else {
+                    const double survival = exp(-is.dist/depth);
+                    absorbed = draw() > survival;
+                }
             }
             if (!hit || absorbed) {
                 kind = MLGPU_ABSORPTION_IN_VOID;
             } else {
-                const double refl = func_eval_tab(fn_pts, fn_off, fn[is.outside ? MLGPU_SURF_OUTER_REFLECTION
-                                                                 : MLGPU_SURF_INNER_REFLECTION], lambda, &err);
+                const double refl = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFLECTION, MLGPU_SURF_INNER_REFLECTION), lambda, &err);
                 if (refl >= draw()) {
                     kind = MLGPU_REFLECTION_ON_SURFACE;
-                    new_s = position(T, is.pos);
-                    new_d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                    s = position(T, is.pos);
+                    d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
                     moved = true;
-                } else if (!(flags & MLGPU_FLAG_TRANSPARENT)) {
+                } else if (!(__ldg(&L->flags) & MLGPU_FLAG_TRANSPARENT)) {
                     kind = MLGPU_ABSORPTION_ON_SURFACE;
                 } else {
                     const v3 inc = orientation_inverse(T, d);
                     const v3 nrm = is.outside ? is.normal : scale(is.normal, -1.0);
-                    const double n_from = func_eval_tab(fn_pts, fn_off, fn[is.outside ? MLGPU_SURF_OUTER_REFRACTION
-                                                                       : MLGPU_SURF_INNER_REFRACTION], lambda, &err);
-                    const double n_to = func_eval_tab(fn_pts, fn_off, fn[is.outside ? MLGPU_SURF_INNER_REFRACTION
-                                                                     : MLGPU_SURF_OUTER_REFRACTION], lambda, &err);
+                    const double n_from = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION), lambda, &err);
+                    const double n_to = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_INNER_REFRACTION, MLGPU_SURF_OUTER_REFRACTION), lambda, &err);
                     const double cosI = dot(nrm, inc)*(-1.0);
                     const double ratio = n_from/n_to;
                     const double sinT2 = ratio*ratio*(1.0 - cosI*cosI);
@@ -363,18 +515,19 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
                     }
                     if (R > draw()) {
                         kind = MLGPU_FRESNEL_REFLECTION_ON_SURFACE;
-                        new_s = position(T, is.pos);
-                        new_d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                        s = position(T, is.pos);
+                        d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
                         moved = true;
                     } else {
                         kind = is.outside ? MLGPU_REFRACTION_TO_INSIDE : MLGPU_REFRACTION_TO_OUTSIDE;
+                        const int32_t flags = __ldg(&L->flags), allowed = __ldg(&L->allowed_node);
                         const bool to_default = is.outside
                             ? (flags & MLGPU_FLAG_INNER_REFRACTION_DEFAULT) != 0
                             : (flags & MLGPU_FLAG_OUTER_REFRACTION_DEFAULT) != 0;
                         root = (allowed >= 0 && !to_default) ? allowed : 0;
                         const v3 refr = add(scale(inc, ratio), scale(nrm, ratio*cosI - cosT));
-                        new_s = position(T, is.pos);
-                        new_d = normalized(orientation(T, refr));
+                        s = position(T, is.pos);
+                        d = normalized(orientation(T, refr));
                         moved = true;
                     }
                 }
@@ -383,7 +536,7 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             {
                 // time-of-flight term, merlict/Photon.cpp:37-56
                 const int32_t f = hit
-                    ? fn[is.outside ? MLGPU_SURF_OUTER_REFRACTION : MLGPU_SURF_INNER_REFRACTION]
+                    ? table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION)
                     : sc.default_refraction;
                 int terr = 0;
                 const double n = func_eval_tab(fn_pts, fn_off, f, lambda, &terr);
@@ -391,45 +544,54 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
                 tof += n*is.dist/299792458.0;
             }
         }
-        const v3 step_start = s;
         n_next = n_int + (count == kNoStep ? 0 : 1);
         survive = moved && (uint32_t)n_next <= max_int;
         if (survive) {
-            s = new_s;
-            d = new_d;
             err = err | (tof_error << 8);
         } else {
-            // the photon ends: its results (Sensor.cpp:14-30,
-            // RayForPropagation.cpp:114-136)
-            const v3 last_world = moved ? new_s : position(T, is.pos);
-            const v3 second_last_world =
-                count == kNoStep ? last_world : (n_int == 1 ? position(IDENTITY, step_start) : step_start);
-            const v3 final_d = moved ? new_d : d;
+            // the photon ends: its results (Sensor.cpp:14-30)
             const int32_t sensor = is.leaf >= 0 ? __ldg(&sc.leaf[is.leaf].sensor) : -1;
             if (sensor >= 0 && tof_error && !err) err = tof_error;
-            v3 inc = mk(0.0, 0.0, 0.0);
-            if (n_next > 1) inc = orientation_inverse(T, normalized(sub(last_world, second_last_world)));
             const DevResults& r = a.results;
             const uint64_t p = (uint64_t)photon;
             r.sensor[p] = sensor;
             if (r.x) static_cast<Out*>(r.x)[p] = (Out)is.pos.x;
             if (r.y) static_cast<Out*>(r.y)[p] = (Out)is.pos.y;
             if (r.time) r.time[p] = tof;
-            if (r.theta_x) static_cast<Out*>(r.theta_x)[p] = (Out)(-1.0*inc.x);
-            if (r.theta_y) static_cast<Out*>(r.theta_y)[p] = (Out)(-1.0*inc.y);
             if (r.final_leaf) r.final_leaf[p] = is.leaf;
             if (r.info)
                 r.info[p] = (uint32_t)kind | ((uint32_t)n_next << 8) |
                     ((k_draw > 255 ? 255u : (uint32_t)k_draw) << 16) | ((uint32_t)err << 24);
-            if (r.final_position) {
-                r.final_position[3*p] = last_world.x;
-                r.final_position[3*p + 1] = last_world.y;
-                r.final_position[3*p + 2] = last_world.z;
-            }
-            if (r.final_direction) {
-                r.final_direction[3*p] = final_d.x;
-                r.final_direction[3*p + 1] = final_d.y;
-                r.final_direction[3*p + 2] = final_d.z;
+            if (r.theta_x || r.theta_y || r.final_position || r.final_direction) {
+                // the last segment (RayForPropagation.cpp:114-136); the
+                // transform and the ray before the step are read again, so
+                // that the step itself need not keep them
+                v3 s0, d0;
+                load_ray(cur, slot, &s0, &d0);
+                if (is.leaf >= 0) {
+#pragma unroll
+                    for (int k = 0; k < 3; k++) load4(sc.leaf[is.leaf].T + 4*k, T + 4*k);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
+                }
+                const v3 last_world = moved ? s : position(T, is.pos);
+                const v3 second_last_world =
+                    count == kNoStep ? last_world : (n_int == 1 ? position(IDENTITY, s0) : s0);
+                v3 inc = mk(0.0, 0.0, 0.0);
+                if (n_next > 1) inc = orientation_inverse(T, normalized(sub(last_world, second_last_world)));
+                if (r.theta_x) static_cast<Out*>(r.theta_x)[p] = (Out)(-1.0*inc.x);
+                if (r.theta_y) static_cast<Out*>(r.theta_y)[p] = (Out)(-1.0*inc.y);
+                if (r.final_position) {
+                    r.final_position[3*p] = last_world.x;
+                    r.final_position[3*p + 1] = last_world.y;
+                    r.final_position[3*p + 2] = last_world.z;
+                }
+                if (r.final_direction) {
+                    r.final_direction[3*p] = d.x;
+                    r.final_direction[3*p + 1] = d.y;
+                    r.final_direction[3*p + 2] = d.z;
+                }
             }
             if (hist)
                 for (uint32_t k = (uint32_t)n_next; k < hist_len; k++)
@@ -452,16 +614,25 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
                 atomicAdd(&w.counters->done[finished_chunk], (unsigned)__popc(same));
         }
     }
-    // warp-ballot compaction of the surviving rays into the next pool
-    const unsigned m = __ballot_sync(kFull, survive);
-    if (m) {
+    // warp-ballot compaction of the surviving rays into the next pool; with
+    // the closest-hit walk, the rays inside a lens from its end, so that the
+    // warps of the next iteration hold rays of one kind
+    int step = kNoStep;
+    if (survive) step = step_kind(a, w, s, d, root);
+    const bool inside = survive && step == kStepTree && w.walk != MLGPU_WALK_LEVELS;
+    const unsigned m = __ballot_sync(kFull, survive && !inside);
+    const unsigned mi = __ballot_sync(kFull, inside);
+    if (m | mi) {
         uint32_t base = 0;
-        if (lane == __ffs(m) - 1) base = atomicAdd(&w.counters->next, (unsigned)__popc(m));
-        base = __shfl_sync(kFull, base, __ffs(m) - 1);
+        if (lane == 0 && m) base = atomicAdd(&w.counters->next, (unsigned)__popc(m));
+        if (lane == 1 && mi) base = atomicAdd(&w.counters->next_inside, (unsigned)__popc(mi));
+        const uint32_t base_m = __shfl_sync(kFull, base, 0), base_i = __shfl_sync(kFull, base, 1);
         if (survive) {
-            const uint32_t o = base + __popc(m & ((1u << lane) - 1u));
-            // the ray as the next iteration takes it: merlict's state, the
-            // cleared closest hit, and what the intake has to queue
+            const unsigned below = (1u << lane) - 1u;
+            const uint32_t o = inside ? w.pool - 1u - (base_i + __popc(mi & below))
+                                      : base_m + __popc(m & below);
+            // the ray as the next iteration takes it: merlict's state and
+            // how it finds its hit
             nxt.photon[o] = photon;
             store_ray(nxt, o, s, d);
             nxt.lambda[o] = lambda;
@@ -470,10 +641,8 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             nxt.n_int[o] = n_next;
             nxt.k_draw[o] = k_draw;
             nxt.err[o] = err;
-            nxt.best_key[o] = kNoKey;
-            nxt.best_leaf[o] = kNoLeaf;
-            nxt.overflow_flag[o] = 0u;
-            nxt.step[o] = prepare_walk(a, nxt, o, s, d, root);
+            if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(sc, nxt, o, s, d, step);
+            nxt.step[o] = step;
         }
     }
 }

@@ -16,26 +16,46 @@
 
 namespace mlgpu {
 
+void launch_wave32_hit(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                       cudaStream_t s) {
+    const int blocks = walk_blocks(w.pool);
+    const size_t smem = closest_hit_smem(a.scene.surf_levels);
+    if (a.in_dtype == MLGPU_F64)
+        wave_hit_kernel<double, kIsectFp32><<<blocks, kWalkThreads, smem, s>>>(a, w, cur);
+    else
+        wave_hit_kernel<float, kIsectFp32><<<blocks, kWalkThreads, smem, s>>>(a, w, cur);
+}
+
+void launch_wave32_tree(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur, int front,
+                        cudaStream_t s) {
+    wave_tree_kernel<kIsectFp32><<<tree_blocks(w.pool), 128, 0, s>>>(a, w, cur, front);
+}
+
+void launch_wave32_resolve(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                           const RayPool& nxt, bool pure, cudaStream_t s) {
+    const int resolve_blocks = (int)((w.pool + kResolveThreads - 1)/kResolveThreads);
+    if (pure) {
+        if (a.out_dtype == MLGPU_F64)
+            wave_resolve_kernel<double, kIsectFp32Pure><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+        else
+            wave_resolve_kernel<float, kIsectFp32Pure><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+    } else {
+        if (a.out_dtype == MLGPU_F64)
+            wave_resolve_kernel<double, kIsectFp32><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+        else
+            wave_resolve_kernel<float, kIsectFp32><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+    }
+}
+
 cudaError_t launch_wave32_isect_resolve(const TraceArgs& a, const WaveBuffers& w,
                                         const RayPool& cur, const RayPool& nxt, bool pure,
                                         cudaStream_t s, cudaEvent_t mid) {
-    const int blocks = (int)((w.pool + 255)/256);
     if (pure) wave_isect_kernel<kIsectFp32Pure><<<w.grid, 256, 0, s>>>(a, w, cur);
     else wave_isect_kernel<kIsectFp32><<<w.grid, 256, 0, s>>>(a, w, cur);
     wave_tie_kernel<<<w.grid, 256, 0, s>>>(w, cur);
     if (mid) cudaEventRecord(mid, s);
     wave_overflow_kernel<<<148, 128, 0, s>>>(a, w, cur);
-    if (pure) {
-        if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp32Pure><<<blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
-        else
-            wave_resolve_kernel<float, kIsectFp32Pure><<<blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
-    } else {
-        if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp32><<<blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
-        else
-            wave_resolve_kernel<float, kIsectFp32><<<blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
-    }
+    launch_wave32_resolve(a, w, cur, nxt, pure, s);
     return cudaGetLastError();
 }
 

@@ -47,55 +47,14 @@ wave_intake_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
     const uint32_t fresh = (uint32_t)(remaining < room ? remaining : room);
     const uint32_t total = active + fresh;
     const uint32_t slot = blockIdx.x*blockDim.x + threadIdx.x;
-    const uint32_t max_int = a.max_interactions;
-    const uint32_t hist_len = max_int + 1;
     bool bvh = false;          // queue the BVH root for this ray
     int nc = 0;                // candidates of a frame-tree walk
     int32_t cand[kTreeCands];
     if (slot < total) {
         int step;
         if (slot >= active) {
-            const uint64_t q = next_input + (slot - active);
-            uint64_t p;
             v3 s, d;
-            double lambda;
-            if (a.sorted) {
-                // the photon's record in tracing order
-                const double2* r = a.sorted + 4*q;
-                const double2 r0 = __ldcg(r), r1 = __ldcg(r + 1), r2 = __ldcg(r + 2),
-                              r3 = __ldcg(r + 3);
-                s = mk(r0.x, r0.y, r1.x);
-                d = normalized(mk(r1.y, r2.x, r2.y));
-                lambda = r3.x;
-                p = (uint64_t)__double_as_longlong(r3.y);
-            } else {
-                p = a.order ? (uint64_t)__ldg(a.order + q) : q;
-                s = mk(load_in<In>(a.photons.sx, p), load_in<In>(a.photons.sy, p),
-                       load_in<In>(a.photons.sz, p));
-                d = normalized(mk(load_in<In>(a.photons.dx, p), load_in<In>(a.photons.dy, p),
-                                  load_in<In>(a.photons.dz, p)));
-                lambda = load_in<In>(a.photons.wavelength, p);
-            }
-            const int32_t root = a.start_node;
-            cur.photon[slot] = (int32_t)p;
-            store_ray(cur, slot, s, d);
-            // Photon::assert_wavelength_is_positive (Photon.cpp:20-28):
-            // merlict throws std::invalid_argument before propagating
-            if (lambda <= 0.0) raise_error(sc.error_word, MLGPU_ERR_INVALID_ARGUMENT);
-            cur.lambda[slot] = lambda;
-            cur.tof[slot] = 0.0;
-            cur.root[slot] = root;
-            cur.n_int[slot] = 1;
-            cur.k_draw[slot] = 0;
-            cur.err[slot] = 0;
-            cur.best_key[slot] = kNoKey;
-            cur.best_leaf[slot] = kNoLeaf;
-            cur.overflow_flag[slot] = 0u;
-            if (a.results.history)
-                store_hist(a.results.history + p*hist_len, s, d, 0.0,
-                           MLGPU_LEAF_PHOTON_SOURCE, MLGPU_PRODUCTION, dot(d, d) < 0.0);
-            step = 1u > max_int ? kNoStep : prepare_walk(a, cur, slot, s, d, root);
-            cur.step[slot] = step;
+            step = admit_photon<In>(a, w, cur, slot, next_input + (slot - active), &s, &d);
         } else {
             step = cur.step[slot];   // prepared by the previous resolve step
         }
@@ -358,99 +317,17 @@ wave_level_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int
     }
 }
 
-// The whole walk of a ray in one thread: a depth-first walk of the BVH with
-// a stack, the same box tests as wave_level_kernel and the same sphere tests
-// as wave_sphere_kernel, so the same candidate leaves; they are queued once
-// per warp after the walk.  A ray whose stack or candidate list fills up
-// goes to merlict's own walk (the overflow kernel).  One thread per ray of
-// the root queue; the ray's FP64 state is read when its first leaf range
-// is hit.
-constexpr int kWalkStack = 3*kMaxBvhLevels + 4;
-constexpr int kWalkCands = 32;
-
-template <bool kF32>
-__global__ void __launch_bounds__(256)
-wave_walk_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
-    const DevScene& sc = a.scene;
-    const uint32_t len = w.counters->level_len[0];
-    const uint32_t n = len < w.level_cap ? len : w.level_cap;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t first = warp_first(); first < n; first += gridDim.x*blockDim.x) {
-        const uint32_t e = first + (uint32_t)lane;
-        uint32_t slot = 0;
-        int32_t cand[kWalkCands];
-        uint32_t nc = 0;
-        bool over = false;
-        if (e < n) {
-            const uint2 q = w.level_q[0][e];
-            slot = q.x;
-            const uint32_t root = q.y;
-            const float4 o = cur.ray_o[slot], iv = cur.ray_i[slot];
-            const float3 dv = make_float3(1.0f/iv.x, 1.0f/iv.y, 1.0f/iv.z);
-            v3 s = mk(0, 0, 0), d = mk(0, 0, 0);
-            double sd = 0.0;
-            bool have_ray = false;
-            int32_t stack[kWalkStack];
-            int sp = 0;
-            stack[sp++] = (int32_t)root;
-            while (sp > 0 && !over) {
-                ChildRefs child;
-                const uint32_t hit = qnode_hits<false>(
-                    reinterpret_cast<const float4*>(sc.bvh_q + stack[--sp]), o, iv, &child);
-                for (int k = kBvhWidth - 1; k >= 0; k--) {
-                    if (!(hit & (1u << k))) continue;
-                    const int32_t ref = child_ref(child, k);
-                    if (ref >= 0) {
-                        if (sp < kWalkStack) stack[sp++] = ref;
-                        else over = true;
-                        continue;
-                    }
-                    const int32_t start = (ref & 0x7fffffff) >> 3;
-                    const int32_t count = (ref & 7) + 1;
-                    if (!kF32 && !have_ray) {
-                        load_ray(cur, slot, &s, &d);
-                        sd = dot(s, d);
-                        have_ray = true;
-                    }
-                    for (int32_t j = start; j < start + count; j++) {
-                        bool pass;
-                        if (kF32) {
-                            pass = sphere_cull32(__ldg(sc.bvh_sphere_f + j), o, dv);
-                        } else {
-                            const double2* c = reinterpret_cast<const double2*>(sc.bvh_sphere + j);
-                            const double2 c01 = __ldg(c), c23 = __ldg(c + 1);
-                            pass = sphere_cull(make_double4(c01.x, c01.y, c23.x, c23.y), s, d, sd);
-                        }
-                        if (pass) {
-                            if (nc < (uint32_t)kWalkCands) cand[nc++] = j;   // the leaf's slot
-                            else over = true;
-                        }
-                    }
-                }
-            }
-        }
-        if (over) {
-            mark_overflow(w, cur, slot);
-            nc = 0;
-        }
-        const uint32_t cb = warp_reserve(&w.counters->isect_len, nc);
-        for (uint32_t k = 0; k < nc; k++) {
-            if (cb + k < w.isect_cap) w.isect_q[cb + k] = make_uint2(slot, (uint32_t)cand[k]);
-            else mark_overflow(w, cur, slot);
-        }
-    }
-}
-
 // counters between the kernels of an iteration
 __global__ void wave_after_intake_kernel(WaveCounters* c, uint32_t pool, uint64_t num_photons,
                                          int fed) {
     const unsigned long long limit = fed ? c->avail_snap : num_photons;
     const unsigned long long remaining = limit - c->next_input;
-    const uint32_t room = pool - c->active;
+    const uint32_t room = pool - c->active - c->inside;
     const uint32_t fresh = (uint32_t)(remaining < room ? remaining : room);
     c->total = c->active + fresh;
     c->next_input += fresh;
     c->next = 0;
+    c->next_inside = 0;
 }
 
 // The value of avail the next iteration admits photons up to: read once
@@ -467,6 +344,7 @@ __global__ void wave_after_resolve_kernel(WaveCounters* c, int fed) {
         if (fed) snapshot_avail(c);
         c->overflow_total += c->overflow_len;
         c->active = c->next;
+        c->inside = c->next_inside;
         c->isect_len = 0;
         c->overflow_len = 0;
     }
@@ -512,23 +390,52 @@ cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* ho
 cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                                   const RayPool& nxt, int form, cudaStream_t s, cudaEvent_t* ev) {
     const int slot_blocks = (int)((w.pool + 255)/256);
+    const int resolve_blocks = (int)((w.pool + kResolveThreads - 1)/kResolveThreads);
     if (ev) cudaEventRecord(ev[0], s);
+    if (w.walk == MLGPU_WALK_STACK) {
+        // intake, walk and intersections in one kernel
+        if (ev) cudaEventRecord(ev[1], s);
+        const int front = a.start_node != 0 || a.scene.surf_levels == 0 ||
+            a.traversal == MLGPU_TRAVERSAL_FRAME_TREE;
+        if (form == MLGPU_TRACER_FP64) {
+            const int blocks = walk_blocks(w.pool);
+            const size_t smem = closest_hit_smem(a.scene.surf_levels);
+            if (a.in_dtype == MLGPU_F64)
+                wave_hit_kernel<double, kIsectFp64><<<blocks, kWalkThreads, smem, s>>>(a, w, cur);
+            else
+                wave_hit_kernel<float, kIsectFp64><<<blocks, kWalkThreads, smem, s>>>(a, w, cur);
+        } else {
+            launch_wave32_hit(a, w, cur, s);
+        }
+        wave_after_intake_kernel<<<1, 1, 0, s>>>(w.counters, w.pool, a.num_photons, a.fed);
+        if (form == MLGPU_TRACER_FP64)
+            wave_tree_kernel<kIsectFp64><<<tree_blocks(w.pool), 128, 0, s>>>(a, w, cur, front);
+        else
+            launch_wave32_tree(a, w, cur, front, s);
+        if (ev) cudaEventRecord(ev[2], s);
+        if (ev) cudaEventRecord(ev[3], s);
+        if (form == MLGPU_TRACER_FP64) {
+            if (a.out_dtype == MLGPU_F64)
+                wave_resolve_kernel<double, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            else
+                wave_resolve_kernel<float, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+        } else {
+            launch_wave32_resolve(a, w, cur, nxt, false, s);
+        }
+        wave_after_resolve_kernel<<<1, 64, 0, s>>>(w.counters, a.fed);
+        if (ev) cudaEventRecord(ev[4], s);
+        return cudaGetLastError();
+    }
     if (a.in_dtype == MLGPU_F64)
         wave_intake_kernel<double><<<slot_blocks, 256, 0, s>>>(a, w, cur);
     else
         wave_intake_kernel<float><<<slot_blocks, 256, 0, s>>>(a, w, cur);
     wave_after_intake_kernel<<<1, 1, 0, s>>>(w.counters, w.pool, a.num_photons, a.fed);
     if (ev) cudaEventRecord(ev[1], s);
-    if (w.walk == MLGPU_WALK_STACK) {
-        if (form == MLGPU_TRACER_FP64) wave_walk_kernel<false><<<w.grid, 256, 0, s>>>(a, w, cur);
-        else wave_walk_kernel<true><<<w.grid, 256, 0, s>>>(a, w, cur);
-    } else {
-        for (int k = 0; k < a.scene.bvh_levels; k++) {
-            const int count = a.scene.bvh_level_start[k + 1] - a.scene.bvh_level_start[k];
-            const int staged = k < w.staged_levels && count <= kMaxStagedNodes ? count : 0;
-            wave_level_kernel<<<w.grid, 256, (size_t)staged*sizeof(QNode), s>>>(a, w, cur, k,
-                                                                                   staged);
-        }
+    for (int k = 0; k < a.scene.bvh_levels; k++) {
+        const int count = a.scene.bvh_level_start[k + 1] - a.scene.bvh_level_start[k];
+        const int staged = k < w.staged_levels && count <= kMaxStagedNodes ? count : 0;
+        wave_level_kernel<<<w.grid, 256, (size_t)staged*sizeof(QNode), s>>>(a, w, cur, k, staged);
     }
     if (ev) cudaEventRecord(ev[2], s);
     if (form == MLGPU_TRACER_FP64) {
@@ -537,9 +444,9 @@ cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, cons
         if (ev) cudaEventRecord(ev[3], s);
         wave_overflow_kernel<<<148, 128, 0, s>>>(a, w, cur);
         if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp64><<<slot_blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<double, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
         else
-            wave_resolve_kernel<float, kIsectFp64><<<slot_blocks, 256, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<float, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
     } else {
         const cudaError_t e = launch_wave32_isect_resolve(a, w, cur, nxt,
                                                           form == MLGPU_TRACER_FP32_PURE, s,

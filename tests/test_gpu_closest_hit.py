@@ -1,0 +1,42 @@
+"""The closest-hit walk (csrc/closest_hit.cuh) at the sizes where its warps
+can go wrong -- fewer rays than a warp, a lane more than a chunk, pools that
+are refilled many times -- against the oracle, bit for bit, with photons
+that are not finite among the others."""
+import numpy as np
+import pytest
+
+from conftest import load_golden
+from merlict_development_kit_b200 import photons as P
+from parity import mismatches
+
+pytestmark = pytest.mark.gpu
+
+
+def batch(name, n):
+    if name == "light_field_small":
+        return P.downward_disc_source(n, 11, 5.55, 21.4, 0.5)
+    return P.isotropic_shell_source(n, 11, 4.0, 2.5)
+
+
+@pytest.mark.parametrize("name", ["primitive_zoo", "light_field_small"])
+@pytest.mark.parametrize("n,pool", [(1, 0), (31, 0), (33, 0), (129, 0), (2049, 1024), (40_001, 1024),
+                                    (70_003, 0), (70_003, 4096)])
+def test_any_number_of_rays(oracle, name, n, pool):
+    from merlict_development_kit_b200 import engine
+    flat, _, _, meta = load_golden(name)
+    ph = batch(name, n)
+    if n > 100:
+        ph["direction_x"][7] = np.nan
+        ph["support_z"][n - 1] = np.inf
+        ph["support_x"][n // 2] = 1e30
+    status, ref, _ = oracle.propagate(flat, ph, meta["max_interactions"], seed=5)
+    assert status == 0
+    scene = engine.Scene(flat)
+    out = scene.propagate(engine.photons_to_device(ph),
+                          engine.PropagationConfig(meta["max_interactions"]), engine.Philox(5),
+                          outputs=("sensor", "x", "y", "time", "theta_x", "theta_y", "final_leaf",
+                                   "info", "final_position", "final_direction"),
+                          tuning={"pool_size": pool, "walk": 2})
+    got = {k: v.cpu().numpy() for k, v in out.items()}
+    assert mismatches(ref, got) == {}
+    scene.close()
