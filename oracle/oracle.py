@@ -49,7 +49,7 @@ def build(reference: bool = True) -> None:
     the reference harness, the sanitizer check of the drop-in's host code
     and (once the engine library is built) the drop-in's test harness."""
     targets = ["oracle"]
-    if reference and os.path.isdir(REFERENCE_DIR):
+    if reference and os.path.isdir(os.path.join(REFERENCE_DIR, "merlict")):
         targets += ["ref", "sanitize"]
         if os.path.exists(ENGINE_SO):
             targets.append("shim")
