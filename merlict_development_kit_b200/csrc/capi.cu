@@ -516,6 +516,10 @@ TraceArgs make_args(const mlgpu_scene* scene, const mlgpu_photons* ph, uint64_t 
 }
 
 constexpr uint32_t kWavePool = 1u << 21;   // ray slots of the wavefront tracers
+// Batches and remainders that one launch takes to their ends (closest-hit
+// walk).
+constexpr uint32_t kFinishBatch = 56832;
+constexpr uint32_t kFinishRays = 56832;
 
 // How the rays of a call find their hits.  One thread per ray through the
 // surface BVH (STACK) unless the caller asks for the level kernels, by name
@@ -527,6 +531,13 @@ int wave_walk(const mlgpu_scene* scene, const mlgpu_settings* st) {
         (scene->dev.surf_levels == 0 && scene->dev.bvh_nodes > 0))
         return MLGPU_WALK_LEVELS;
     return MLGPU_WALK_STACK;
+}
+
+// Bytes of the property tables in shared memory, 0 if they do not fit.
+int table_smem_bytes(const mlgpu_scene* scene) {
+    const size_t bytes = (size_t)scene->dev.num_fn_points*3*sizeof(double) +
+        ((size_t)scene->dev.num_functions + 1)*sizeof(int32_t);
+    return bytes <= 16384 ? (int)bytes : 0;
 }
 
 // Carves the two ray pools, the candidate lists and the counters out of
@@ -575,9 +586,7 @@ int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32
     w->isect_dist = reinterpret_cast<double*>(take(isect_cap*8));
     w->isect_cap = (uint32_t)isect_cap;
     w->overflow = reinterpret_cast<uint32_t*>(take(P*4));
-    const size_t fn_bytes = (size_t)scene->dev.num_fn_points*3*sizeof(double) +
-        ((size_t)scene->dev.num_functions + 1)*sizeof(int32_t);
-    w->fn_smem_bytes = fn_bytes <= 16384 ? (int)fn_bytes : 0;
+    w->fn_smem_bytes = table_smem_bytes(scene);
     return MLGPU_OK;
 }
 
@@ -688,6 +697,30 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     WaveBuffers w;
     RayPool pools[2];
     const int walk = wave_walk(scene, st);
+    // the FP32 forms' double-precision parts are contracted as the compiler
+    // sees fit: a second kernel would round them differently
+    const bool finish = walk == MLGPU_WALK_STACK && form == MLGPU_TRACER_FP64;
+    if (finish && !feed && a.num_photons <= std::min(kFinishBatch, want)) {
+        // a batch that one launch takes to its end
+        std::memset(&w, 0, sizeof(w));
+        std::memset(&pools[0], 0, sizeof(pools[0]));
+        w.walk = walk;
+        w.fn_smem_bytes = table_smem_bytes(scene);
+        Profiler::Chain ch;
+        const bool timed = scene->prof.on && scene->prof.take(2, ch.ev);
+        if (timed) cudaEventRecord(ch.ev[0], stream);
+        const cudaError_t e = launch_wave_finish(a, w, pools[0], true, pool, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
+        scene->launches++;
+        if (timed) {
+            cudaEventRecord(ch.ev[1], stream);
+            ch.n = 2; ch.cls[0] = MLGPU_KERNEL_PLAIN; ch.launches[0] = 1;
+            scene->prof.add(ch);
+        }
+        scene->wave_stats.calls++;
+        scene->wave_stats.iterations++;
+        return MLGPU_OK;
+    }
     const int rc = wave_buffers(scene, pool, st->grid_blocks, st->staged_levels,
                                 st->queue_capacity, walk, &w, &pools[0], &pools[1]);
     if (rc) return rc;
@@ -735,13 +768,20 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     const int walk_launches = stack ? 1 : scene->dev.bvh_levels;
     const int iteration_launches = stack ? 5 : walk_launches + 7;
     uint64_t iteration = 0;
+    bool more = a.num_photons > pool;   // photons wait for slots
     while (true) {
         if (graph) {
             MLGPU_CUDA(cudaGraphLaunch(scene->wave_graph, stream));
             iteration += (uint64_t)period;
             scene->launches += (uint64_t)period*(uint64_t)iteration_launches + 1;
         } else {
-            for (int g = 0; g < period; g++, iteration++) {
+            // Without a period of the caller's own the closest-hit walk looks
+            // after the first iteration of a batch that fits the pool, and
+            // after every second once the input is used up: few rays may be
+            // left then, and one launch ends them.
+            const int steps = !finish || st->check_period > 0 || more ? period
+                : iteration == 0 ? 1 : 2;
+            for (int g = 0; g < steps; g++, iteration++) {
                 const RayPool& cur = pools[iteration & 1];
                 const RayPool& nxt = pools[(iteration + 1) & 1];
                 Profiler::Chain ch;
@@ -785,7 +825,21 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
                 scene->launches++;
             }
         }
-        if (h.active + h.inside == 0 && h.next_input >= a.num_photons) break;
+        more = h.next_input < a.num_photons;
+        const uint32_t left = h.active + h.inside;
+        if (left == 0 && h.next_input >= a.num_photons) break;
+        if (finish && left <= kFinishRays && h.next_input >= a.num_photons) {
+            // the last rays, in one launch
+            const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], false, left, stream);
+            if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
+            scene->launches++;
+            for (int c = 0; feed && c < feed->pieces; c++) {
+                if (downloaded[c]) continue;
+                const int r = feed->download(c);
+                if (r) return r;
+            }
+            break;
+        }
         if (iteration > bound)
             return fail(MLGPU_ERR_RUNTIME, "wavefront tracer did not drain its pool");
     }

@@ -53,6 +53,7 @@ constexpr unsigned long long kNoKey = ~0ull;
 
 constexpr int kWalkThreads = 128;
 constexpr int kWalkBlocks = 4;   // resident per SM
+constexpr int kFinishBlocks = 3;
 constexpr int kLists = 3;
 constexpr int kLeafList = 96;                  // leaves a list holds
 static_assert(kLeafList >= 32 + kBvhWidth, "a list of fewer than 32 takes any one group's leaves");
@@ -78,6 +79,13 @@ inline size_t closest_hit_smem(int levels) {
 inline int walk_blocks(uint32_t rays) {
     const uint32_t need = (rays + kWalkThreads - 1)/kWalkThreads;
     return (int)(need < 148u*kWalkBlocks ? need : 148u*kWalkBlocks);
+}
+
+// Blocks of a launch that takes at most `rays` rays to their ends: a warp
+// per ray up to a full GPU.
+inline int finish_blocks(uint32_t rays) {
+    const uint32_t need = (rays + kWalkThreads/32 - 1)/(kWalkThreads/32);
+    return (int)(need < 148u*kFinishBlocks ? need : 148u*kFinishBlocks);
 }
 
 inline int tree_blocks(uint32_t rays) {
@@ -329,6 +337,32 @@ __device__ __forceinline__ uint32_t work_off(const DevScene& sc, WalkWarp* w, in
         nq -= k;
     }
     return (uint32_t)n | (uint32_t)np << 10 | (uint32_t)nq << 20;
+}
+
+// One visit of every lane that walks; the groups of leaves reached join the
+// queue.  Returns the groups queued.  All lanes of the warp call it, with
+// fewer than 32 groups queued.
+__device__ __forceinline__ int visit_nodes(const DevScene& sc, WalkWarp* w, uint32_t* stack,
+                                           int lane, int groups, WalkLane* l) {
+    uint2 group = make_uint2(0u, 0u);
+    if (l->walking) group = walk_step(sc, l, stack);
+    const unsigned reached = __ballot_sync(kFull, (group.x & 0xffu) != 0);
+    if ((group.x & 0xffu) != 0)
+        w->group[groups + __popc(reached & ((1u << lane) - 1u))] =
+            make_uint2(group.x, group.y | (uint32_t)lane << 24);
+    __syncwarp();
+    return groups + __popc(reached);
+}
+
+// Intersects queued leaves while there are 32 groups, or 32 leaves of a
+// kind; with `all`, every one.
+template <int kIsect>
+__device__ __forceinline__ void intersect_queued(const DevScene& sc, WalkWarp* w, int lane, bool all,
+                                                 int* groups, uint32_t* listed, WalkLane* l) {
+    while (*groups >= 32 || (all && (*groups | (int)*listed) != 0)) {
+        *groups = spread_groups(w, lane, *groups, listed);
+        *listed = work_off<kIsect>(sc, w, lane, *listed, all && *groups == 0 ? 1 : 32, l);
+    }
 }
 
 // The closest hit in the frame subtree `root` by merlict's own walk of its

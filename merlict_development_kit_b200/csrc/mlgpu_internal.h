@@ -327,6 +327,11 @@ struct WaveBuffers {
 // it, after the BVH walk, after the intersections and after the resolve step.
 cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                                   const RayPool& nxt, int form, cudaStream_t s, cudaEvent_t* ev);
+// One launch that takes the pool's rays and the photons that have not set
+// out to their ends; with `batch`, the whole batch without a pool.  `rays`:
+// at most so many.  Closest-hit walk of the FP64 form only.
+cudaError_t launch_wave_finish(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                               bool batch, uint32_t rays, cudaStream_t s);
 // The counters to `host`: the device address of pinned host memory.
 cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* host,
                                          cudaStream_t s);

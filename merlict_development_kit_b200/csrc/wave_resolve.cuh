@@ -138,54 +138,89 @@ __device__ __forceinline__ void prepare_levels(const DevScene& sc, const RayPool
     p.ray_i[slot] = make_float4(1.0f/fdx, 1.0f/fdy, 1.0f/fdz, 0.0f);
 }
 
-// A new photon into slot `slot`: the next of the batch's tracing order
-// (merlict::Photon's constructor, Ray.cpp:16-20, RayForPropagation.cpp:52-64),
-// prepared like the survivors the previous resolve step prepared.  Returns
-// its step.
+// A photon between interactions (a merlict Photon: its ray, what its history
+// adds up to, its random stream).
+struct PhotonRay {
+    v3 s, d;
+    double lambda, tof;
+    int32_t photon, root, n_int, k_draw;
+    int32_t err;             // error | time-of-flight error << 8
+};
+
+__device__ __forceinline__ void load_photon(const RayPool& cur, uint32_t slot, PhotonRay* q) {
+    load_ray(cur, slot, &q->s, &q->d);
+    q->photon = cur.photon[slot];
+    q->lambda = cur.lambda[slot];
+    q->tof = cur.tof[slot];
+    q->root = cur.root[slot];
+    q->n_int = cur.n_int[slot];
+    q->k_draw = cur.k_draw[slot];
+    q->err = cur.err[slot];
+}
+
+// Photon q of the batch's tracing order as it sets out (merlict::Photon's
+// constructor, Ray.cpp:16-20, RayForPropagation.cpp:52-64).  Returns its step.
 template <typename In>
-__device__ __forceinline__ int admit_photon(const TraceArgs& a, const WaveBuffers& w,
-                                            const RayPool& cur, uint32_t slot, uint64_t q,
-                                            v3* support, v3* direction) {
+__device__ __forceinline__ int start_photon(const TraceArgs& a, const WaveBuffers& w, uint64_t q,
+                                            PhotonRay* out) {
     const uint32_t max_int = a.max_interactions;
     uint64_t p;
-    v3 s, d;
-    double lambda;
     if (a.sorted) {
         // the photon's record in tracing order
         const double2* r = a.sorted + 4*q;
         const double2 r0 = __ldcg(r), r1 = __ldcg(r + 1), r2 = __ldcg(r + 2), r3 = __ldcg(r + 3);
-        s = mk(r0.x, r0.y, r1.x);
-        d = normalized_rn(mk(r1.y, r2.x, r2.y));
-        lambda = r3.x;
+        out->s = mk(r0.x, r0.y, r1.x);
+        out->d = normalized_rn(mk(r1.y, r2.x, r2.y));
+        out->lambda = r3.x;
         p = (uint64_t)__double_as_longlong(r3.y);
     } else {
         p = a.order ? (uint64_t)__ldg(a.order + q) : q;
-        s = mk(load_in<In>(a.photons.sx, p), load_in<In>(a.photons.sy, p),
-               load_in<In>(a.photons.sz, p));
-        d = normalized_rn(mk(load_in<In>(a.photons.dx, p), load_in<In>(a.photons.dy, p),
-                          load_in<In>(a.photons.dz, p)));
-        lambda = load_in<In>(a.photons.wavelength, p);
+        out->s = mk(load_in<In>(a.photons.sx, p), load_in<In>(a.photons.sy, p),
+                    load_in<In>(a.photons.sz, p));
+        out->d = normalized_rn(mk(load_in<In>(a.photons.dx, p), load_in<In>(a.photons.dy, p),
+                                  load_in<In>(a.photons.dz, p)));
+        out->lambda = load_in<In>(a.photons.wavelength, p);
     }
-    const int32_t root = a.start_node;
-    cur.photon[slot] = (int32_t)p;
-    store_ray(cur, slot, s, d);
+    out->photon = (int32_t)p;
     // Photon::assert_wavelength_is_positive (Photon.cpp:20-28): merlict
     // throws std::invalid_argument before propagating
-    if (lambda <= 0.0) raise_error(a.scene.error_word, MLGPU_ERR_INVALID_ARGUMENT);
-    cur.lambda[slot] = lambda;
-    cur.tof[slot] = 0.0;
-    cur.root[slot] = root;
-    cur.n_int[slot] = 1;
-    cur.k_draw[slot] = 0;
-    cur.err[slot] = 0;
+    if (out->lambda <= 0.0) raise_error(a.scene.error_word, MLGPU_ERR_INVALID_ARGUMENT);
+    out->tof = 0.0;
+    out->root = a.start_node;
+    out->n_int = 1;
+    out->k_draw = 0;
+    out->err = 0;
     if (a.results.history)
-        store_hist(a.results.history + p*(max_int + 1), s, d, 0.0, MLGPU_LEAF_PHOTON_SOURCE,
-                   MLGPU_PRODUCTION, dot(d, d) < 0.0);
-    const int step = 1u > max_int ? kNoStep : step_kind(a, w, s, d, root);
-    if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(a.scene, cur, slot, s, d, step);
-    cur.step[slot] = step;
-    *support = s;
-    *direction = d;
+        store_hist(a.results.history + p*(max_int + 1), out->s, out->d, 0.0,
+                   MLGPU_LEAF_PHOTON_SOURCE, MLGPU_PRODUCTION, dot(out->d, out->d) < 0.0);
+    return 1u > max_int ? kNoStep : step_kind(a, w, out->s, out->d, out->root);
+}
+
+__device__ __forceinline__ void store_photon(const RayPool& p, uint32_t slot, const PhotonRay& q,
+                                             int step) {
+    p.photon[slot] = q.photon;
+    store_ray(p, slot, q.s, q.d);
+    p.lambda[slot] = q.lambda;
+    p.tof[slot] = q.tof;
+    p.root[slot] = q.root;
+    p.n_int[slot] = q.n_int;
+    p.k_draw[slot] = q.k_draw;
+    p.err[slot] = q.err;
+    p.step[slot] = step;
+}
+
+// The same into slot `slot` of the pool, prepared like the survivors the
+// previous resolve step prepared.
+template <typename In>
+__device__ __forceinline__ int admit_photon(const TraceArgs& a, const WaveBuffers& w,
+                                            const RayPool& cur, uint32_t slot, uint64_t q,
+                                            v3* support, v3* direction) {
+    PhotonRay ray;
+    const int step = start_photon<In>(a, w, q, &ray);
+    if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(a.scene, cur, slot, ray.s, ray.d, step);
+    store_photon(cur, slot, ray, step);
+    *support = ray.s;
+    *direction = ray.d;
     return step;
 }
 
@@ -230,10 +265,7 @@ wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
         const unsigned idle = __ballot_sync(kFull, !l.walking);
         const int free_lanes = __popc(idle);
         const bool refill = free_lanes == 32 || (free_lanes >= kRefill && chunk < chunks);
-        while (groups >= 32 || (refill && (groups | (int)listed) != 0)) {
-            groups = spread_groups(sw, lane, groups, &listed);
-            listed = work_off<kIsect>(sc, sw, lane, listed, refill && groups == 0 ? 1 : 32, &l);
-        }
+        intersect_queued<kIsect>(sc, sw, lane, refill, &groups, &listed, &l);
         if (refill) {
             const bool is_free = (idle >> lane) & 1u;
             if (is_free && have) {
@@ -266,14 +298,7 @@ wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
             if (taken == 32) { chunk += stride; taken = 0; }
             __syncwarp();
         }
-        uint2 group = make_uint2(0u, 0u);
-        if (l.walking) group = walk_step(sc, &l, stack);
-        const unsigned reached = __ballot_sync(kFull, (group.x & 0xffu) != 0);
-        if ((group.x & 0xffu) != 0)
-            sw->group[groups + __popc(reached & ((1u << lane) - 1u))] =
-                make_uint2(group.x, group.y | (uint32_t)lane << 24);
-        groups += __popc(reached);
-        __syncwarp();
+        groups = visit_nodes(sc, sw, stack, lane, groups, &l);
     }
 }
 
@@ -360,8 +385,326 @@ wave_overflow_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) 
     }
 }
 
-// Three blocks per SM (80 registers, a few hundred bytes spilled): measured
-// faster than two blocks at 126 registers.
+// The photon's step to the hit found for it, `best` (kNoLeaf: none) at
+// best_dist: the intersection, the interaction with the surface
+// (merlict/PhotonAndFrame.cpp:13-124), the history entry and the
+// time-of-flight term.  Returns true if the photon goes on, then with its
+// new ray; else its results are written.  `before` reads the ray before the
+// step again where the results ask for it.
+template <typename Out, int kIsect, typename Before>
+__device__ __forceinline__ bool resolve_photon(const TraceArgs& a, const double* fn_pts,
+                                               const int32_t* fn_off, int step, int32_t best,
+                                               double best_dist, PhotonRay* q, Before before) {
+    const DevScene& sc = a.scene;
+    const uint32_t max_int = a.max_interactions;
+    const uint32_t hist_len = max_int + 1;
+    v3& s = q->s;
+    v3& d = q->d;
+    const double lambda = q->lambda;
+    double& tof = q->tof;
+    int32_t& root = q->root;
+    int32_t& k_draw = q->k_draw;
+    const int32_t photon = q->photon, n_int = q->n_int;
+    int err = q->err & 0xff;
+    int tof_error = (q->err >> 8) & 0xff;
+    const uint64_t stream = a.rng.photon_offset + (uint64_t)photon;
+    mlgpu_history_entry* hist =
+        a.results.history ? a.results.history + (uint64_t)photon*hist_len : nullptr;
+
+    Isec is;
+    int kind = MLGPU_PRODUCTION;
+    bool moved = false;      // then s and d are the photon's new ray
+    double T[12];
+    if (step == kNoStep) {
+        is.leaf = MLGPU_LEAF_PHOTON_SOURCE;
+        is.pos = s; is.normal = d; is.dist = 0.0; is.outside = dot(d, d) < 0.0;
+#pragma unroll
+        for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
+    } else {
+        // merlict's closest hit among the candidates: minimum distance,
+        // ties to merlict's visiting order (RayAndFrame.cpp:160-173)
+        {
+            // the winner of the search at its distance; the FP32 forms
+            // intersect it again with the hit point refined
+            if (best == kNoLeaf) {
+                set_void(&is, s, d);
+            } else if (kIsect == kIsectFp64) {
+                hit_at(sc, best, best_dist, s, d, T, &is);
+            } else {
+                const fp32::Hit32 h = fp32::intersect32<true>(sc, best, fp32::dmk(s.x, s.y, s.z),
+                                                        fp32::dmk(d.x, d.y, d.z),
+                                                        kIsect == kIsectFp32Pure);
+                if (h.leaf < 0) {
+                    set_void(&is, s, d);
+                } else {
+                    is.leaf = h.leaf;
+                    is.pos = mk(h.p.x, h.p.y, h.p.z);
+                    is.normal = mk(h.n.x, h.n.y, h.n.z);
+                    is.dist = h.v;
+                    is.outside = h.outside;
+                }
+            }
+        }
+        const bool hit = is.leaf >= 0;
+        const LeafRec* L = hit ? sc.leaf + is.leaf : nullptr;
+        if (hit && kIsect != kIsectFp64) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) load4(L->T + 4*k, T + 4*k);
+        } else if (!hit) {
+#pragma unroll
+            for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
+        }
+        // a property table of the surface, by the side the ray comes from
+        auto table = [&](int outside, int inside) {
+            return __ldg(L->fn + (is.outside ? outside : inside));
+        };
+        auto draw = [&]() -> double {
+            const uint32_t k = (uint32_t)k_draw++;
+            if (a.rng.mode == MLGPU_RNG_REPLAY) {
+                if (k >= a.rng.stride) { if (!err) err = MLGPU_ERR_RUNTIME; return 0.5; }
+                return __ldg(a.rng.uniforms + (uint64_t)photon*a.rng.stride + k);
+            }
+            return mlgpu_philox_uniform(a.rng.seed, stream, k);
+        };
+        bool absorbed = false;
+        if (hit) {
+            // absorbed_in_medium_before_reaching_surface, PhotonAndFrame.cpp:32-38
+            const double depth = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_ABSORPTION, MLGPU_SURF_INNER_ABSORPTION), lambda, &err);
+            if (depth != depth && a.rng.mode == MLGPU_RNG_PHILOX) {
+                // merlict's default table evaluates to NaN, and no draw
+                // is larger than that: only the draw is counted
+                k_draw++;
+            } else {
+                const double survival = exp(-is.dist/depth);
+                absorbed = draw() > survival;
+            }
+        }
+        if (!hit || absorbed) {
+            kind = MLGPU_ABSORPTION_IN_VOID;
+        } else {
+            const double refl = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFLECTION, MLGPU_SURF_INNER_REFLECTION), lambda, &err);
+            if (refl >= draw()) {
+                kind = MLGPU_REFLECTION_ON_SURFACE;
+                s = position(T, is.pos);
+                d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                moved = true;
+            } else if (!(__ldg(&L->flags) & MLGPU_FLAG_TRANSPARENT)) {
+                kind = MLGPU_ABSORPTION_ON_SURFACE;
+            } else {
+                const v3 inc = orientation_inverse(T, d);
+                const v3 nrm = is.outside ? is.normal : scale(is.normal, -1.0);
+                const double n_from = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION), lambda, &err);
+                const double n_to = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_INNER_REFRACTION, MLGPU_SURF_OUTER_REFRACTION), lambda, &err);
+                const double cosI = dot(nrm, inc)*(-1.0);
+                const double ratio = n_from/n_to;
+                const double sinT2 = ratio*ratio*(1.0 - cosI*cosI);
+                const double cosT = sqrt(1.0 - sinT2);
+                double R;
+                if (sinT2 > 1.0) {
+                    R = 1.0;
+                } else {
+                    const double rOrth = (n_from*cosI - n_to*cosT) / (n_from*cosI + n_to*cosT);
+                    const double rPar = (n_to*cosI - n_from*cosT) / (n_to*cosI + n_from*cosT);
+                    R = (rOrth*rOrth + rPar*rPar) / 2.0;
+                }
+                if (R > draw()) {
+                    kind = MLGPU_FRESNEL_REFLECTION_ON_SURFACE;
+                    s = position(T, is.pos);
+                    d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                    moved = true;
+                } else {
+                    kind = is.outside ? MLGPU_REFRACTION_TO_INSIDE : MLGPU_REFRACTION_TO_OUTSIDE;
+                    const int32_t flags = __ldg(&L->flags), allowed = __ldg(&L->allowed_node);
+                    const bool to_default = is.outside
+                        ? (flags & MLGPU_FLAG_INNER_REFRACTION_DEFAULT) != 0
+                        : (flags & MLGPU_FLAG_OUTER_REFRACTION_DEFAULT) != 0;
+                    root = (allowed >= 0 && !to_default) ? allowed : 0;
+                    const v3 refr = add(scale(inc, ratio), scale(nrm, ratio*cosI - cosT));
+                    s = position(T, is.pos);
+                    d = normalized(orientation(T, refr));
+                    moved = true;
+                }
+            }
+        }
+        if (hist) store_hist(&hist[n_int], is.pos, is.normal, is.dist, is.leaf, kind, is.outside);
+        {
+            // time-of-flight term, merlict/Photon.cpp:37-56
+            const int32_t f = hit
+                ? table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION)
+                : sc.default_refraction;
+            int terr = 0;
+            const double n = func_eval_tab(fn_pts, fn_off, f, lambda, &terr);
+            if (terr && !tof_error) tof_error = terr;
+            tof += n*is.dist/299792458.0;
+        }
+    }
+    const int32_t n_next = n_int + (step == kNoStep ? 0 : 1);
+    const bool survive = moved && (uint32_t)n_next <= max_int;
+    q->n_int = n_next;
+    if (survive) {
+        q->err = err | (tof_error << 8);
+    } else {
+        // the photon ends: its results (Sensor.cpp:14-30)
+        const int32_t sensor = is.leaf >= 0 ? __ldg(&sc.leaf[is.leaf].sensor) : -1;
+        if (sensor >= 0 && tof_error && !err) err = tof_error;
+        const DevResults& r = a.results;
+        const uint64_t p = (uint64_t)photon;
+        r.sensor[p] = sensor;
+        if (r.x) static_cast<Out*>(r.x)[p] = (Out)is.pos.x;
+        if (r.y) static_cast<Out*>(r.y)[p] = (Out)is.pos.y;
+        if (r.time) r.time[p] = tof;
+        if (r.final_leaf) r.final_leaf[p] = is.leaf;
+        if (r.info)
+            r.info[p] = (uint32_t)kind | ((uint32_t)n_next << 8) |
+                ((k_draw > 255 ? 255u : (uint32_t)k_draw) << 16) | ((uint32_t)err << 24);
+        if (r.theta_x || r.theta_y || r.final_position || r.final_direction) {
+            // the last segment (RayForPropagation.cpp:114-136); the
+            // transform and the ray before the step are read again, so
+            // that the step itself need not keep them
+            v3 s0, d0;
+            before(&s0, &d0);
+            if (is.leaf >= 0) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) load4(sc.leaf[is.leaf].T + 4*k, T + 4*k);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
+            }
+            const v3 last_world = moved ? s : position(T, is.pos);
+            const v3 second_last_world =
+                step == kNoStep ? last_world : (n_int == 1 ? position(IDENTITY, s0) : s0);
+            v3 inc = mk(0.0, 0.0, 0.0);
+            if (n_next > 1) inc = orientation_inverse(T, normalized(sub(last_world, second_last_world)));
+            if (r.theta_x) static_cast<Out*>(r.theta_x)[p] = (Out)(-1.0*inc.x);
+            if (r.theta_y) static_cast<Out*>(r.theta_y)[p] = (Out)(-1.0*inc.y);
+            if (r.final_position) {
+                r.final_position[3*p] = last_world.x;
+                r.final_position[3*p + 1] = last_world.y;
+                r.final_position[3*p + 2] = last_world.z;
+            }
+            if (r.final_direction) {
+                r.final_direction[3*p] = d.x;
+                r.final_direction[3*p + 1] = d.y;
+                r.final_direction[3*p + 2] = d.z;
+            }
+        }
+        if (hist)
+            for (uint32_t k = (uint32_t)n_next; k < hist_len; k++)
+                store_hist(&hist[k], mk(0, 0, 0), mk(0, 0, 0), 0.0, MLGPU_LEAF_PHOTON_SOURCE, 0, false);
+        if (err) raise_error(sc.error_word, (unsigned int)err);
+    }
+    return survive;
+}
+
+// The property tables, staged in shared memory when they fit.
+__device__ __forceinline__ void stage_tables(const DevScene& sc, int bytes, double* s_fn,
+                                             const double** pts, const int32_t** off) {
+    *pts = sc.fn_points;
+    *off = sc.fn_offset;
+    if (!bytes) return;
+    const int np = 3*sc.num_fn_points;
+    int32_t* s_off = reinterpret_cast<int32_t*>(s_fn + np);
+    for (int k = threadIdx.x; k < np; k += blockDim.x) s_fn[k] = __ldg(sc.fn_points + k);
+    for (int k = threadIdx.x; k <= sc.num_functions; k += blockDim.x) s_off[k] = __ldg(sc.fn_offset + k);
+    __syncthreads();
+    *pts = s_fn;
+    *off = s_off;
+}
+
+// Photons from where they are to their ends, in one launch: the rays of the
+// pool and, up to the batch's end, photons that have not set out (with
+// `batch`: the whole batch, no pool).  A warp keeps its photons, one per
+// lane, and alternates between searching their hits and resolving them; no
+// host, no counters and no other kernel come between the interactions of a
+// photon.  For few rays that is what counts: a wavefront iteration is four
+// launches however few rays it advances.  With fewer photons than the grid
+// has lanes each warp takes fewer, since a warp lasts as long as its longest
+// photon.
+template <typename In, typename Out>
+__global__ void __launch_bounds__(kWalkThreads, kFinishBlocks)
+wave_finish_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int batch) {
+    extern __shared__ double2 s_walk[];
+    const DevScene& sc = a.scene;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kWalkThreads/32;
+    WalkWarp* sw = reinterpret_cast<WalkWarp*>(s_walk) + warp;
+    uint32_t* stacks = reinterpret_cast<uint32_t*>(reinterpret_cast<WalkWarp*>(s_walk) + kWarps);
+    uint32_t* stack = stacks + threadIdx.x;
+    const double* fn_pts;
+    const int32_t* fn_off;
+    stage_tables(sc, w.fn_smem_bytes,
+                 reinterpret_cast<double*>(stacks + kWalkThreads*sc.surf_levels), &fn_pts, &fn_off);
+    const uint32_t active = batch ? 0u : w.counters->active;
+    const uint32_t inside = batch ? 0u : w.counters->inside;
+    const unsigned long long next_input = batch ? 0ull : w.counters->next_input;
+    const uint32_t front = active + (uint32_t)(a.num_photons - next_input);
+    const uint32_t rays = front + inside;
+    const uint32_t warps = gridDim.x*kWarps;
+    const uint32_t share = (rays + warps - 1)/warps, per = share < 32u ? share : 32u;
+    WalkLane l;
+    l.eps = 0.0f;
+    l.key = kNoKey;
+    for (uint32_t first = (blockIdx.x*kWarps + warp)*per; first < rays; first += warps*per) {
+        const uint32_t index = first + (uint32_t)lane;
+        bool live = (uint32_t)lane < per && index < rays;
+        PhotonRay q;
+        int step = kNoStep;
+        if (live) {
+            const uint32_t slot = index < front ? index : w.pool - 1u - (index - front);
+            if (index >= active && index < front) {
+                step = start_photon<In>(a, w, next_input + (index - active), &q);
+            } else {
+                load_photon(cur, slot, &q);
+                step = cur.step[slot];
+            }
+        }
+        while (__any_sync(kFull, live)) {
+            uint32_t listed = 0;
+            int groups = 0;
+            l.walking = false;
+            if (live) {
+                if (step == kStepBvh) {
+                    walk_begin(sc, q.s, q.d, sw, lane, &l);
+                } else {
+                    sw->ray[0][lane] = make_double2(q.s.x, q.s.y);
+                    sw->ray[1][lane] = make_double2(q.s.z, q.d.x);
+                    sw->ray[2][lane] = make_double2(q.d.y, q.d.z);
+                }
+            }
+            __syncwarp();
+            while (true) {
+                const bool walking = __any_sync(kFull, l.walking);
+                intersect_queued<kIsectFp64>(sc, sw, lane, !walking, &groups, &listed, &l);
+                if (!walking) break;
+                groups = visit_nodes(sc, sw, stack, lane, groups, &l);
+            }
+            int32_t best = kNoLeaf;
+            double dist = 0.0;
+            if (live && step == kStepBvh) {
+                best = sw->leaf[lane];
+                dist = __longlong_as_double((long long)sw->key[lane]);
+            }
+            if (live && step == kStepTree)
+                best = closest_hit_tree<kIsectFp64>(sc, q.root, q.s, q.d, &dist);
+            if (live) {
+                live = resolve_photon<Out, kIsectFp64>(
+                    a, fn_pts, fn_off, step, best, dist, &q, [&](v3* s, v3* d) {
+                        const double2 x = sw->ray[0][lane], y = sw->ray[1][lane],
+                                      z = sw->ray[2][lane];
+                        *s = mk(x.x, x.y, y.x);
+                        *d = mk(y.y, z.x, z.y);
+                    });
+                if (live) step = step_kind(a, w, q.s, q.d, q.root);
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// 72 registers, seven blocks of 128 per SM: the step waits on its gathers and
+// on chains of double-precision arithmetic, so more warps win over fewer
+// spills (four blocks without spills 4.8 ms per 1e7 photons on the
+// light-field telescope, five to eight blocks 4.5, 4.4, 4.3, 4.3).
 constexpr int kResolveThreads = 128;
 constexpr int kResolveBlocks = 7;
 
@@ -369,239 +712,29 @@ template <typename Out, int kIsect>
 __global__ void __launch_bounds__(kResolveThreads, kResolveBlocks)
 wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, const RayPool nxt) {
     const DevScene& sc = a.scene;
-    // the property tables, staged in shared memory when they fit
     extern __shared__ double s_fn[];
-    const double* fn_pts = sc.fn_points;
-    const int32_t* fn_off = sc.fn_offset;
-    if (w.fn_smem_bytes) {
-        const int np = 3*sc.num_fn_points;
-        int32_t* s_off = reinterpret_cast<int32_t*>(s_fn + np);
-        for (int k = threadIdx.x; k < np; k += blockDim.x) s_fn[k] = __ldg(sc.fn_points + k);
-        for (int k = threadIdx.x; k <= sc.num_functions; k += blockDim.x) s_off[k] = __ldg(sc.fn_offset + k);
-        __syncthreads();
-        fn_pts = s_fn;
-        fn_off = s_off;
-    }
+    const double* fn_pts;
+    const int32_t* fn_off;
+    stage_tables(sc, w.fn_smem_bytes, s_fn, &fn_pts, &fn_off);
     const uint32_t total = w.counters->total;
     const uint32_t index = blockIdx.x*blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const bool valid = index < total + w.counters->inside;
     const uint32_t slot = index < total ? index : w.pool - 1u - (index - total);
-    const uint32_t max_int = a.max_interactions;
-    const uint32_t hist_len = max_int + 1;
 
     bool survive = false;
     int32_t finished_chunk = -1;   // fed propagation: the chunk of a photon that ends here
-    // state of this slot after the step (written to the next pool if it survives)
-    int32_t photon = 0, root = 0, n_next = 0, k_draw = 0, err = 0;
-    v3 s = mk(0, 0, 0), d = mk(0, 0, 0);
-    double lambda = 0.0, tof = 0.0;
-    int32_t count = 0;
+    PhotonRay q;
     if (valid) {
-        load_ray(cur, slot, &s, &d);
-        count = cur.step[slot];
-    }
-
-    if (valid) {
-        photon = cur.photon[slot];
-        lambda = cur.lambda[slot];
-        tof = cur.tof[slot];
-        root = cur.root[slot];
-        const int32_t n_int = cur.n_int[slot];
-        k_draw = cur.k_draw[slot];
-        const int32_t err_word = cur.err[slot];
-        err = err_word & 0xff;
-        int tof_error = (err_word >> 8) & 0xff;
-        const uint64_t stream = a.rng.photon_offset + (uint64_t)photon;
-        mlgpu_history_entry* hist =
-            a.results.history ? a.results.history + (uint64_t)photon*hist_len : nullptr;
-
-        Isec is;
-        int kind = MLGPU_PRODUCTION;
-        bool moved = false;      // then s and d are the photon's new ray
-        double T[12];
-        if (count == kNoStep) {
-            is.leaf = MLGPU_LEAF_PHOTON_SOURCE;
-            is.pos = s; is.normal = d; is.dist = 0.0; is.outside = dot(d, d) < 0.0;
-#pragma unroll
-            for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
-        } else {
-            // merlict's closest hit among the candidates: minimum distance,
-            // ties to merlict's visiting order (RayAndFrame.cpp:160-173)
-            {
-                // the winner of the search at its distance; the FP32 forms
-                // intersect it again with the hit point refined
-                const int32_t best = cur.best_leaf[slot];
-                if (best == kNoLeaf) {
-                    set_void(&is, s, d);
-                } else if (kIsect == kIsectFp64) {
-                    hit_at(sc, best, __longlong_as_double((long long)cur.best_key[slot]), s, d, T, &is);
-                } else {
-                    const fp32::Hit32 h = fp32::intersect32<true>(sc, best, fp32::dmk(s.x, s.y, s.z),
-                                                            fp32::dmk(d.x, d.y, d.z),
-                                                            kIsect == kIsectFp32Pure);
-                    if (h.leaf < 0) {
-                        set_void(&is, s, d);
-                    } else {
-                        is.leaf = h.leaf;
-                        is.pos = mk(h.p.x, h.p.y, h.p.z);
-                        is.normal = mk(h.n.x, h.n.y, h.n.z);
-                        is.dist = h.v;
-                        is.outside = h.outside;
-                    }
-                }
-            }
-            const bool hit = is.leaf >= 0;
-            const LeafRec* L = hit ? sc.leaf + is.leaf : nullptr;
-            if (hit && kIsect != kIsectFp64) {
-#pragma unroll
-                for (int k = 0; k < 3; k++) load4(L->T + 4*k, T + 4*k);
-            } else if (!hit) {
-#pragma unroll
-                for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
-            }
-            // a property table of the surface, by the side the ray comes from
-            auto table = [&](int outside, int inside) {
-                return __ldg(L->fn + (is.outside ? outside : inside));
-            };
-            auto draw = [&]() -> double {
-                const uint32_t k = (uint32_t)k_draw++;
-                if (a.rng.mode == MLGPU_RNG_REPLAY) {
-                    if (k >= a.rng.stride) { if (!err) err = MLGPU_ERR_RUNTIME; return 0.5; }
-                    return __ldg(a.rng.uniforms + (uint64_t)photon*a.rng.stride + k);
-                }
-                return mlgpu_philox_uniform(a.rng.seed, stream, k);
-            };
-            bool absorbed = false;
-            if (hit) {
-                // absorbed_in_medium_before_reaching_surface, PhotonAndFrame.cpp:32-38
-                const double depth = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_ABSORPTION, MLGPU_SURF_INNER_ABSORPTION), lambda, &err);
-                if (depth != depth && a.rng.mode == MLGPU_RNG_PHILOX) {
-                    // merlict's default table evaluates to NaN, and no draw
-                    // is larger than that: only the draw is counted
-                    k_draw++;
-                } else {
-                    const double survival = exp(-is.dist/depth);
-                    absorbed = draw() > survival;
-                }
-            }
-            if (!hit || absorbed) {
-                kind = MLGPU_ABSORPTION_IN_VOID;
-            } else {
-                const double refl = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFLECTION, MLGPU_SURF_INNER_REFLECTION), lambda, &err);
-                if (refl >= draw()) {
-                    kind = MLGPU_REFLECTION_ON_SURFACE;
-                    s = position(T, is.pos);
-                    d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
-                    moved = true;
-                } else if (!(__ldg(&L->flags) & MLGPU_FLAG_TRANSPARENT)) {
-                    kind = MLGPU_ABSORPTION_ON_SURFACE;
-                } else {
-                    const v3 inc = orientation_inverse(T, d);
-                    const v3 nrm = is.outside ? is.normal : scale(is.normal, -1.0);
-                    const double n_from = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION), lambda, &err);
-                    const double n_to = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_INNER_REFRACTION, MLGPU_SURF_OUTER_REFRACTION), lambda, &err);
-                    const double cosI = dot(nrm, inc)*(-1.0);
-                    const double ratio = n_from/n_to;
-                    const double sinT2 = ratio*ratio*(1.0 - cosI*cosI);
-                    const double cosT = sqrt(1.0 - sinT2);
-                    double R;
-                    if (sinT2 > 1.0) {
-                        R = 1.0;
-                    } else {
-                        const double rOrth = (n_from*cosI - n_to*cosT) / (n_from*cosI + n_to*cosT);
-                        const double rPar = (n_to*cosI - n_from*cosT) / (n_to*cosI + n_from*cosT);
-                        R = (rOrth*rOrth + rPar*rPar) / 2.0;
-                    }
-                    if (R > draw()) {
-                        kind = MLGPU_FRESNEL_REFLECTION_ON_SURFACE;
-                        s = position(T, is.pos);
-                        d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
-                        moved = true;
-                    } else {
-                        kind = is.outside ? MLGPU_REFRACTION_TO_INSIDE : MLGPU_REFRACTION_TO_OUTSIDE;
-                        const int32_t flags = __ldg(&L->flags), allowed = __ldg(&L->allowed_node);
-                        const bool to_default = is.outside
-                            ? (flags & MLGPU_FLAG_INNER_REFRACTION_DEFAULT) != 0
-                            : (flags & MLGPU_FLAG_OUTER_REFRACTION_DEFAULT) != 0;
-                        root = (allowed >= 0 && !to_default) ? allowed : 0;
-                        const v3 refr = add(scale(inc, ratio), scale(nrm, ratio*cosI - cosT));
-                        s = position(T, is.pos);
-                        d = normalized(orientation(T, refr));
-                        moved = true;
-                    }
-                }
-            }
-            if (hist) store_hist(&hist[n_int], is.pos, is.normal, is.dist, is.leaf, kind, is.outside);
-            {
-                // time-of-flight term, merlict/Photon.cpp:37-56
-                const int32_t f = hit
-                    ? table(MLGPU_SURF_OUTER_REFRACTION, MLGPU_SURF_INNER_REFRACTION)
-                    : sc.default_refraction;
-                int terr = 0;
-                const double n = func_eval_tab(fn_pts, fn_off, f, lambda, &terr);
-                if (terr && !tof_error) tof_error = terr;
-                tof += n*is.dist/299792458.0;
-            }
-        }
-        n_next = n_int + (count == kNoStep ? 0 : 1);
-        survive = moved && (uint32_t)n_next <= max_int;
-        if (survive) {
-            err = err | (tof_error << 8);
-        } else {
-            // the photon ends: its results (Sensor.cpp:14-30)
-            const int32_t sensor = is.leaf >= 0 ? __ldg(&sc.leaf[is.leaf].sensor) : -1;
-            if (sensor >= 0 && tof_error && !err) err = tof_error;
-            const DevResults& r = a.results;
-            const uint64_t p = (uint64_t)photon;
-            r.sensor[p] = sensor;
-            if (r.x) static_cast<Out*>(r.x)[p] = (Out)is.pos.x;
-            if (r.y) static_cast<Out*>(r.y)[p] = (Out)is.pos.y;
-            if (r.time) r.time[p] = tof;
-            if (r.final_leaf) r.final_leaf[p] = is.leaf;
-            if (r.info)
-                r.info[p] = (uint32_t)kind | ((uint32_t)n_next << 8) |
-                    ((k_draw > 255 ? 255u : (uint32_t)k_draw) << 16) | ((uint32_t)err << 24);
-            if (r.theta_x || r.theta_y || r.final_position || r.final_direction) {
-                // the last segment (RayForPropagation.cpp:114-136); the
-                // transform and the ray before the step are read again, so
-                // that the step itself need not keep them
-                v3 s0, d0;
-                load_ray(cur, slot, &s0, &d0);
-                if (is.leaf >= 0) {
-#pragma unroll
-                    for (int k = 0; k < 3; k++) load4(sc.leaf[is.leaf].T + 4*k, T + 4*k);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 12; k++) T[k] = IDENTITY[k];
-                }
-                const v3 last_world = moved ? s : position(T, is.pos);
-                const v3 second_last_world =
-                    count == kNoStep ? last_world : (n_int == 1 ? position(IDENTITY, s0) : s0);
-                v3 inc = mk(0.0, 0.0, 0.0);
-                if (n_next > 1) inc = orientation_inverse(T, normalized(sub(last_world, second_last_world)));
-                if (r.theta_x) static_cast<Out*>(r.theta_x)[p] = (Out)(-1.0*inc.x);
-                if (r.theta_y) static_cast<Out*>(r.theta_y)[p] = (Out)(-1.0*inc.y);
-                if (r.final_position) {
-                    r.final_position[3*p] = last_world.x;
-                    r.final_position[3*p + 1] = last_world.y;
-                    r.final_position[3*p + 2] = last_world.z;
-                }
-                if (r.final_direction) {
-                    r.final_direction[3*p] = d.x;
-                    r.final_direction[3*p + 1] = d.y;
-                    r.final_direction[3*p + 2] = d.z;
-                }
-            }
-            if (hist)
-                for (uint32_t k = (uint32_t)n_next; k < hist_len; k++)
-                    store_hist(&hist[k], mk(0, 0, 0), mk(0, 0, 0), 0.0, MLGPU_LEAF_PHOTON_SOURCE, 0, false);
-            if (err) raise_error(sc.error_word, (unsigned int)err);
-            if (a.fed) {
-                int32_t c = 0;
-                while (c + 1 < a.feed_chunks && p >= a.feed_start[c + 1]) c++;
-                finished_chunk = c;
-            }
+        load_photon(cur, slot, &q);
+        survive = resolve_photon<Out, kIsect>(
+            a, fn_pts, fn_off, cur.step[slot], cur.best_leaf[slot],
+            kIsect == kIsectFp64 ? __longlong_as_double((long long)cur.best_key[slot]) : 0.0, &q,
+            [&](v3* s, v3* d) { load_ray(cur, slot, s, d); });
+        if (!survive && a.fed) {
+            int32_t c = 0;
+            while (c + 1 < a.feed_chunks && (uint64_t)q.photon >= a.feed_start[c + 1]) c++;
+            finished_chunk = c;
         }
     }
     // fed propagation: finished photons per chunk, one addition per chunk
@@ -618,7 +751,7 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
     // the closest-hit walk, the rays inside a lens from its end, so that the
     // warps of the next iteration hold rays of one kind
     int step = kNoStep;
-    if (survive) step = step_kind(a, w, s, d, root);
+    if (survive) step = step_kind(a, w, q.s, q.d, q.root);
     const bool inside = survive && step == kStepTree && w.walk != MLGPU_WALK_LEVELS;
     const unsigned m = __ballot_sync(kFull, survive && !inside);
     const unsigned mi = __ballot_sync(kFull, inside);
@@ -633,16 +766,8 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
                                       : base_m + __popc(m & below);
             // the ray as the next iteration takes it: merlict's state and
             // how it finds its hit
-            nxt.photon[o] = photon;
-            store_ray(nxt, o, s, d);
-            nxt.lambda[o] = lambda;
-            nxt.tof[o] = tof;
-            nxt.root[o] = root;
-            nxt.n_int[o] = n_next;
-            nxt.k_draw[o] = k_draw;
-            nxt.err[o] = err;
-            if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(sc, nxt, o, s, d, step);
-            nxt.step[o] = step;
+            store_photon(nxt, o, q, step);
+            if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(sc, nxt, o, q.s, q.d, step);
         }
     }
 }

@@ -458,6 +458,24 @@ cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, cons
     return cudaGetLastError();
 }
 
+cudaError_t launch_wave_finish(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
+                               bool batch, uint32_t rays, cudaStream_t s) {
+    WaveBuffers v = w;
+    size_t smem = closest_hit_smem(a.scene.surf_levels);
+    if (smem + (size_t)v.fn_smem_bytes > 49152) v.fn_smem_bytes = 0;   // tables from global memory
+    smem += (size_t)v.fn_smem_bytes;
+    const int blocks = finish_blocks(rays);
+    if (a.in_dtype == MLGPU_F64 && a.out_dtype == MLGPU_F64)
+        wave_finish_kernel<double, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+    else if (a.in_dtype == MLGPU_F64)
+        wave_finish_kernel<double, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+    else if (a.out_dtype == MLGPU_F64)
+        wave_finish_kernel<float, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+    else
+        wave_finish_kernel<float, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+    return cudaGetLastError();
+}
+
 int wave_persistent_blocks() {
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
