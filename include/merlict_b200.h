@@ -259,8 +259,11 @@ enum { MLGPU_WALK_DEFAULT = 0, MLGPU_WALK_LEVELS = 1, MLGPU_WALK_STACK = 2 };
 
 /* photon_order: COHERENT sorts the batch by a 4-D cell key of support and
  * direction before tracing, so that neighbouring ray slots follow nearly
- * the same path (results are the same in any order).  DEFAULT is COHERENT
- * for batches of at least 65,536 photons and INPUT below.                  */
+ * the same path (results are the same in any order).  DEFAULT is INPUT for
+ * the STACK walk on device buffers, which gains no more from the order than
+ * the sort costs; for the LEVELS walk, the work-queue tracer and the
+ * host-buffer calls it is COHERENT for batches of at least 65,536 photons
+ * and INPUT below.                                                         */
 enum { MLGPU_ORDER_DEFAULT = 0, MLGPU_ORDER_INPUT = 1, MLGPU_ORDER_COHERENT = 2 };
 
 typedef struct mlgpu_scene mlgpu_scene;

@@ -516,10 +516,6 @@ TraceArgs make_args(const mlgpu_scene* scene, const mlgpu_photons* ph, uint64_t 
 }
 
 constexpr uint32_t kWavePool = 1u << 21;   // ray slots of the wavefront tracers
-// Batches and remainders that one launch takes to their ends (closest-hit
-// walk).
-constexpr uint32_t kFinishBatch = 56832;
-constexpr uint32_t kFinishRays = 56832;
 
 // How the rays of a call find their hits.  One thread per ray through the
 // surface BVH (STACK) unless the caller asks for the level kernels, by name
@@ -540,6 +536,15 @@ int table_smem_bytes(const mlgpu_scene* scene) {
     return bytes <= 16384 ? (int)bytes : 0;
 }
 
+// The pinned copy of the counters.
+int wave_host_counters(mlgpu_scene* scene) {
+    if (!scene->wave_host) MLGPU_CUDA(cudaMallocHost(&scene->wave_host, sizeof(WaveCounters)));
+    if (!scene->wave_host_dev)
+        MLGPU_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&scene->wave_host_dev),
+                                            scene->wave_host, 0));
+    return MLGPU_OK;
+}
+
 // Carves the two ray pools, the candidate lists and the counters out of
 // one device buffer.
 int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32_t queue_cap,
@@ -553,10 +558,8 @@ int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32
     const size_t per_pool = up(P*48) + 3*up(P*8) + 8*up(P*4) + 2*up(P*16);
     const size_t rest = 2*up(level_cap*8) + up(isect_cap*8) + up(isect_cap*8) + up(P*4);
     MLGPU_CUDA(scene->wave.reserve(kWaveCounterBytes + 2*per_pool + rest));
-    if (!scene->wave_host) MLGPU_CUDA(cudaMallocHost(&scene->wave_host, sizeof(WaveCounters)));
-    if (!scene->wave_host_dev)
-        MLGPU_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&scene->wave_host_dev),
-                                            scene->wave_host, 0));
+    const int rc = wave_host_counters(scene);
+    if (rc) return rc;
     if (!scene->wave_grid) scene->wave_grid = wave_persistent_blocks();
     char* b = static_cast<char*>(scene->wave.ptr);
     w->counters = reinterpret_cast<WaveCounters*>(b);
@@ -679,48 +682,97 @@ struct FeedPlan {
     std::function<int(int)> download;
 };
 
+// What comes before the wavefront of an FP64 batch in the input order: a
+// batch small enough for one launch is traced by it (*done); of a larger
+// one, the photons that miss the scenery end in a first look, and if few are
+// left, one launch ends those as well; else they are a's photons, by index,
+// when this returns.  The input order is the default: sorting 1e7 photons of
+// the light-field telescope takes 1.2 ms and gains the walk as much (18.22
+// against 18.30 ms), smaller and sparser batches lose by it (80,000 photons
+// 467 against 563 us, 25e6 photons of air showers 3.8 against 5.6 ms, 8e6 of
+// the large reflector in FP32 5.3 against 6.2 ms).
+int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, cudaStream_t stream, bool* done) {
+    WaveBuffers w;
+    RayPool none;
+    std::memset(&w, 0, sizeof(w));
+    std::memset(&none, 0, sizeof(none));
+    w.walk = MLGPU_WALK_STACK;
+    w.fn_smem_bytes = table_smem_bytes(scene);
+    const uint64_t n = a->num_photons;
+    const bool whole = n <= std::min(kFinishRays, want);
+    if (!whole && n >= (1ull << 31)) return MLGPU_OK;
+    Profiler::Chain ch;
+    const bool timed = scene->prof.on && scene->prof.take(2, ch.ev);
+    if (timed) cudaEventRecord(ch.ev[0], stream);
+    cudaError_t e;
+    if (whole) {
+        e = launch_wave_finish(*a, w, none, kFinishBatchMode, (uint32_t)n, stream);
+    } else {
+        const int rc = wave_host_counters(scene);
+        if (rc) return rc;
+        MLGPU_CUDA(scene->order.reserve(256 + kWaveCounterBytes + 4*n));
+        char* b = static_cast<char*>(scene->order.ptr);
+        w.counters = reinterpret_cast<WaveCounters*>(b);
+        w.first = reinterpret_cast<uint32_t*>(b + kWaveCounterBytes);
+        MLGPU_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(WaveCounters), stream));
+        e = launch_wave_first(*a, w, stream);
+        if (e == cudaSuccess && want >= kFinishRays) {
+            TraceArgs l = *a;
+            l.order = w.first;
+            e = launch_wave_finish(l, w, none, kFinishListMode, kFinishRays, stream);
+            scene->launches++;
+        }
+        if (e == cudaSuccess)
+            e = launch_wave_counters_to_host(w.counters, scene->wave_host_dev, stream);
+        scene->launches++;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
+    scene->launches++;
+    if (timed) {
+        cudaEventRecord(ch.ev[1], stream);
+        ch.n = 2; ch.cls[0] = MLGPU_KERNEL_PLAIN; ch.launches[0] = 1;
+        scene->prof.add(ch);
+    }
+    *done = whole;
+    if (!whole) {
+        MLGPU_CUDA(cudaStreamSynchronize(stream));
+        const uint64_t listed = scene->wave_host->avail_snap;
+        *done = listed == 0 || (want >= kFinishRays && listed <= kFinishRays);
+        a->num_photons = listed;
+        a->order = w.first;
+    }
+    if (*done) {
+        scene->wave_stats.calls++;
+        scene->wave_stats.iterations++;
+    }
+    return MLGPU_OK;
+}
+
 int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
                   cudaStream_t stream, const FeedPlan* feed = nullptr) {
     const int form = st->tracer;
+    const int walk = wave_walk(scene, st);
+    // the FP32 forms' double-precision parts are contracted as the compiler
+    // sees fit: a second kernel would round them differently
+    const bool finish = walk == MLGPU_WALK_STACK && form == MLGPU_TRACER_FP64;
+    const uint32_t want = st->pool_size ? st->pool_size : kWavePool;
     if (feed) {
         a.sorted = feed->records;
         a.order = nullptr;
         a.fed = 1;
         a.feed_chunks = feed->pieces;
         for (int c = 0; c <= feed->pieces; c++) a.feed_start[c] = feed->start[c];
-    } else {
+    } else if (finish && st->photon_order != MLGPU_ORDER_COHERENT) {
+        bool done = false;
+        const int r = first_look(scene, &a, want, stream, &done);
+        if (r || done) return r;
+    } else if (walk != MLGPU_WALK_STACK || st->photon_order == MLGPU_ORDER_COHERENT) {
         const int ro = tracing_order(scene, &a, st, stream, true);
         if (ro) return ro;
     }
-    const uint32_t want = st->pool_size ? st->pool_size : kWavePool;
     const uint32_t pool = (uint32_t)std::min<uint64_t>(a.num_photons, want);
     WaveBuffers w;
     RayPool pools[2];
-    const int walk = wave_walk(scene, st);
-    // the FP32 forms' double-precision parts are contracted as the compiler
-    // sees fit: a second kernel would round them differently
-    const bool finish = walk == MLGPU_WALK_STACK && form == MLGPU_TRACER_FP64;
-    if (finish && !feed && a.num_photons <= std::min(kFinishBatch, want)) {
-        // a batch that one launch takes to its end
-        std::memset(&w, 0, sizeof(w));
-        std::memset(&pools[0], 0, sizeof(pools[0]));
-        w.walk = walk;
-        w.fn_smem_bytes = table_smem_bytes(scene);
-        Profiler::Chain ch;
-        const bool timed = scene->prof.on && scene->prof.take(2, ch.ev);
-        if (timed) cudaEventRecord(ch.ev[0], stream);
-        const cudaError_t e = launch_wave_finish(a, w, pools[0], true, pool, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
-        scene->launches++;
-        if (timed) {
-            cudaEventRecord(ch.ev[1], stream);
-            ch.n = 2; ch.cls[0] = MLGPU_KERNEL_PLAIN; ch.launches[0] = 1;
-            scene->prof.add(ch);
-        }
-        scene->wave_stats.calls++;
-        scene->wave_stats.iterations++;
-        return MLGPU_OK;
-    }
     const int rc = wave_buffers(scene, pool, st->grid_blocks, st->staged_levels,
                                 st->queue_capacity, walk, &w, &pools[0], &pools[1]);
     if (rc) return rc;
@@ -830,7 +882,8 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
         if (left == 0 && h.next_input >= a.num_photons) break;
         if (finish && left <= kFinishRays && h.next_input >= a.num_photons) {
             // the last rays, in one launch
-            const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], false, left, stream);
+            const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], kFinishPoolMode, left,
+                                                     stream);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
             scene->launches++;
             for (int c = 0; feed && c < feed->pieces; c++) {

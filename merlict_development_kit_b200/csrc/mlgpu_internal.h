@@ -318,7 +318,16 @@ struct WaveBuffers {
     double* isect_dist;      // distance to each candidate's hit, -1: none
     uint32_t isect_cap;
     uint32_t* overflow;      // [pool] slots for merlict's own walk
+    uint32_t* first;         // photons that the first look lists for the tracer
 };
+
+// Batches, lists and remainders that one launch takes to their ends: a lane
+// each on the full GPU (148 SMs of three blocks).  Measured on the
+// light-field telescope: the wavefront is 30-60 us slower for batches up to
+// this size; remainders of up to 8,000, 28,000, 56,832, 120,000 and 250,000
+// rays make 1e6 photons 2.40, 2.40, 2.39, 2.39 and 2.51 ms.
+constexpr uint32_t kFinishRays = 56832;
+enum { kFinishPoolMode = 0, kFinishBatchMode = 1, kFinishListMode = 2 };
 
 // One iteration of a wavefront tracer: walk, queue and intersect the
 // candidates, resolve.  `form` is MLGPU_TRACER_FP64, _FP32 or _FP32_PURE;
@@ -327,11 +336,13 @@ struct WaveBuffers {
 // it, after the BVH walk, after the intersections and after the resolve step.
 cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                                   const RayPool& nxt, int form, cudaStream_t s, cudaEvent_t* ev);
-// One launch that takes the pool's rays and the photons that have not set
-// out to their ends; with `batch`, the whole batch without a pool.  `rays`:
-// at most so many.  Closest-hit walk of the FP64 form only.
+// One launch that takes photons to their ends, at most `rays` (`mode`:
+// wave_finish_kernel).  Closest-hit walk of the FP64 form only.
 cudaError_t launch_wave_finish(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
-                               bool batch, uint32_t rays, cudaStream_t s);
+                               int mode, uint32_t rays, cudaStream_t s);
+// The first look at a batch: ends the photons that miss the scenery and
+// lists the others in w.first, their number in the counters' avail_snap.
+cudaError_t launch_wave_first(const TraceArgs& a, const WaveBuffers& w, cudaStream_t s);
 // The counters to `host`: the device address of pinned host memory.
 cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* host,
                                          cudaStream_t s);

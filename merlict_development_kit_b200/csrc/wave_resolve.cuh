@@ -611,9 +611,63 @@ __device__ __forceinline__ void stage_tables(const DevScene& sc, int bytes, doub
     *off = s_off;
 }
 
+// The first look at a large batch: a photon that misses the root frame's
+// sphere (most of an air shower's) ends here, its void result written where
+// it is read, and the others' indices are listed in w.first for the tracer,
+// so that only they pass through the pool.  Streams the planes once: 25e6
+// photons of air showers, 2 % of which are listed, took 5.6 ms through the
+// pool in coherent order and 3.8 ms in input order.
+template <typename In, typename Out>
+__global__ void __launch_bounds__(256, 4)
+wave_first_kernel(const TraceArgs a, const WaveBuffers w) {
+    extern __shared__ double s_fn[];
+    const double* fn_pts;
+    const int32_t* fn_off;
+    stage_tables(a.scene, w.fn_smem_bytes, s_fn, &fn_pts, &fn_off);
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t)gridDim.x*8;
+    // a warp looks at kRun x 32 consecutive photons per turn: one addition to
+    // the list's length for all of them
+    constexpr int kRun = 4;
+    for (uint64_t first = ((uint64_t)blockIdx.x*8 + (threadIdx.x >> 5))*(32*kRun);
+         first < a.num_photons; first += warps*(32*kRun)) {
+        unsigned listed[kRun];
+        uint32_t sum = 0;
+#pragma unroll
+        for (int r = 0; r < kRun; r++) {
+            const uint64_t i = first + 32u*r + (uint64_t)lane;
+            bool on = false;
+            if (i < a.num_photons) {
+                PhotonRay q;
+                const int step = start_photon<In>(a, w, i, &q);
+                on = step == kStepBvh || step == kStepTree;
+                if (!on) {
+                    const v3 s = q.s, d = q.d;
+                    resolve_photon<Out, kIsectFp64>(a, fn_pts, fn_off, step, kNoLeaf, 0.0, &q,
+                                                    [&](v3* s0, v3* d0) { *s0 = s; *d0 = d; });
+                }
+            }
+            listed[r] = __ballot_sync(kFull, on);
+            sum += (uint32_t)__popc(listed[r]);
+        }
+        if (sum == 0) continue;
+        uint32_t at = 0;
+        if (lane == 0) at = (uint32_t)atomicAdd(&w.counters->avail_snap, (unsigned long long)sum);
+        at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+        for (int r = 0; r < kRun; r++) {
+            if ((listed[r] >> lane) & 1u)
+                w.first[at + __popc(listed[r] & ((1u << lane) - 1u))] =
+                    (uint32_t)(first + 32u*r) + (uint32_t)lane;
+            at += (uint32_t)__popc(listed[r]);
+        }
+    }
+}
+
 // Photons from where they are to their ends, in one launch: the rays of the
-// pool and, up to the batch's end, photons that have not set out (with
-// `batch`: the whole batch, no pool).  A warp keeps its photons, one per
+// pool and, up to the batch's end, photons that have not set out.  Without a
+// pool (kFinishBatchMode), the whole batch; with kFinishListMode, the photons
+// that wave_first_kernel listed, unless there are more than kFinishRays.  A warp keeps its photons, one per
 // lane, and alternates between searching their hits and resolving them; no
 // host, no counters and no other kernel come between the interactions of a
 // photon.  For few rays that is what counts: a wavefront iteration is four
@@ -622,7 +676,7 @@ __device__ __forceinline__ void stage_tables(const DevScene& sc, int bytes, doub
 // photon.
 template <typename In, typename Out>
 __global__ void __launch_bounds__(kWalkThreads, kFinishBlocks)
-wave_finish_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int batch) {
+wave_finish_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int mode) {
     extern __shared__ double2 s_walk[];
     const DevScene& sc = a.scene;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -634,10 +688,13 @@ wave_finish_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, in
     const int32_t* fn_off;
     stage_tables(sc, w.fn_smem_bytes,
                  reinterpret_cast<double*>(stacks + kWalkThreads*sc.surf_levels), &fn_pts, &fn_off);
-    const uint32_t active = batch ? 0u : w.counters->active;
-    const uint32_t inside = batch ? 0u : w.counters->inside;
-    const unsigned long long next_input = batch ? 0ull : w.counters->next_input;
-    const uint32_t front = active + (uint32_t)(a.num_photons - next_input);
+    const bool pool = mode == kFinishPoolMode;
+    const uint32_t active = pool ? w.counters->active : 0u;
+    const uint32_t inside = pool ? w.counters->inside : 0u;
+    const unsigned long long next_input = pool ? w.counters->next_input : 0ull;
+    const unsigned long long input = mode == kFinishListMode ? w.counters->avail_snap : a.num_photons;
+    if (mode == kFinishListMode && input > kFinishRays) return;
+    const uint32_t front = active + (uint32_t)(input - next_input);
     const uint32_t rays = front + inside;
     const uint32_t warps = gridDim.x*kWarps;
     const uint32_t share = (rays + warps - 1)/warps, per = share < 32u ? share : 32u;

@@ -459,20 +459,35 @@ cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, cons
 }
 
 cudaError_t launch_wave_finish(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
-                               bool batch, uint32_t rays, cudaStream_t s) {
+                               int mode, uint32_t rays, cudaStream_t s) {
     WaveBuffers v = w;
     size_t smem = closest_hit_smem(a.scene.surf_levels);
     if (smem + (size_t)v.fn_smem_bytes > 49152) v.fn_smem_bytes = 0;   // tables from global memory
     smem += (size_t)v.fn_smem_bytes;
     const int blocks = finish_blocks(rays);
     if (a.in_dtype == MLGPU_F64 && a.out_dtype == MLGPU_F64)
-        wave_finish_kernel<double, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+        wave_finish_kernel<double, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, mode);
     else if (a.in_dtype == MLGPU_F64)
-        wave_finish_kernel<double, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+        wave_finish_kernel<double, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, mode);
     else if (a.out_dtype == MLGPU_F64)
-        wave_finish_kernel<float, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+        wave_finish_kernel<float, double><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, mode);
     else
-        wave_finish_kernel<float, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, batch);
+        wave_finish_kernel<float, float><<<blocks, kWalkThreads, smem, s>>>(a, v, cur, mode);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_wave_first(const TraceArgs& a, const WaveBuffers& w, cudaStream_t s) {
+    const uint64_t tiles = (a.num_photons + 255)/256;
+    const int blocks = (int)(tiles < 148u*8u ? tiles : 148u*8u);
+    const size_t smem = (size_t)w.fn_smem_bytes;
+    if (a.in_dtype == MLGPU_F64 && a.out_dtype == MLGPU_F64)
+        wave_first_kernel<double, double><<<blocks, 256, smem, s>>>(a, w);
+    else if (a.in_dtype == MLGPU_F64)
+        wave_first_kernel<double, float><<<blocks, 256, smem, s>>>(a, w);
+    else if (a.out_dtype == MLGPU_F64)
+        wave_first_kernel<float, double><<<blocks, 256, smem, s>>>(a, w);
+    else
+        wave_first_kernel<float, float><<<blocks, 256, smem, s>>>(a, w);
     return cudaGetLastError();
 }
 

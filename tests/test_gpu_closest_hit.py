@@ -13,6 +13,8 @@ pytestmark = pytest.mark.gpu
 
 
 def batch(name, n):
+    if name == "sparse":      # most miss the telescope: ended by the first look
+        return P.downward_disc_source(n, 11, 60.0, 21.4, 0.5)
     if name == "light_field_small":
         return P.downward_disc_source(n, 11, 5.55, 21.4, 0.5)
     return P.isotropic_shell_source(n, 11, 4.0, 2.5)
@@ -22,9 +24,18 @@ def batch(name, n):
 @pytest.mark.parametrize("n,pool", [(1, 0), (31, 0), (33, 0), (129, 0), (2049, 1024), (40_001, 1024),
                                     (70_003, 0), (70_003, 4096)])
 def test_any_number_of_rays(oracle, name, n, pool):
+    check(oracle, name, batch(name, n), pool)
+
+
+@pytest.mark.parametrize("n,pool,order", [(100_003, 0, 0), (100_003, 1024, 0), (100_003, 0, 2)])
+def test_a_sparse_batch(oracle, n, pool, order):
+    check(oracle, "light_field_small", batch("sparse", n), pool, order)
+
+
+def check(oracle, name, ph, pool, order=0):
     from merlict_development_kit_b200 import engine
     flat, _, _, meta = load_golden(name)
-    ph = batch(name, n)
+    n = len(ph["wavelength"])
     if n > 100:
         ph["direction_x"][7] = np.nan
         ph["support_z"][n - 1] = np.inf
@@ -36,7 +47,7 @@ def test_any_number_of_rays(oracle, name, n, pool):
                           engine.PropagationConfig(meta["max_interactions"]), engine.Philox(5),
                           outputs=("sensor", "x", "y", "time", "theta_x", "theta_y", "final_leaf",
                                    "info", "final_position", "final_direction"),
-                          tuning={"pool_size": pool, "walk": 2})
+                          tuning={"pool_size": pool, "walk": 2, "photon_order": order})
     got = {k: v.cpu().numpy() for k, v in out.items()}
     assert mismatches(ref, got) == {}
     scene.close()
