@@ -231,7 +231,8 @@ typedef struct mlgpu_settings {
     int32_t tracer;         /* MLGPU_TRACER_*                                 */
     int32_t block_size;     /* 0 = default                                    */
     int32_t traversal;      /* MLGPU_TRAVERSAL_*                              */
-    uint32_t pool_size;     /* ray slots of the wavefront pool (2^21)         */
+    uint32_t pool_size;     /* ray slots of the wavefront pool (2^23; 2^21 for
+                               the LEVELS walk and the host-buffer calls)      */
     int32_t check_period;   /* iterations between host checks of the pool (4) */
     int32_t use_graph;      /* 1: each check period is one CUDA-graph launch  */
     int32_t grid_blocks;    /* blocks of the grid-stride kernels (8 per SM)   */

@@ -515,7 +515,13 @@ TraceArgs make_args(const mlgpu_scene* scene, const mlgpu_photons* ph, uint64_t 
     return a;
 }
 
-constexpr uint32_t kWavePool = 1u << 21;   // ray slots of the wavefront tracers
+// Ray slots of the wavefront tracers: for the level kernels, whose queues
+// hold 24 entries per slot, and for a fed propagation; and for the
+// closest-hit walk, where every iteration costs some 60 us of ends of
+// kernels (1e7 photons of the light-field telescope with 2^20, 2^21, 2^22
+// and 2^23 slots: 19.1, 17.6, 17.1 and 16.9 ms).
+constexpr uint32_t kWavePool = 1u << 21;
+constexpr uint32_t kWalkPool = 1u << 23;
 
 // How the rays of a call find their hits.  One thread per ray through the
 // surface BVH (STACK) unless the caller asks for the level kernels, by name
@@ -555,8 +561,9 @@ int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32
     const bool queues = walk == MLGPU_WALK_LEVELS;
     const size_t level_cap = !queues ? 0 : queue_cap ? queue_cap : 8*P;
     const size_t isect_cap = !queues ? 0 : queue_cap ? queue_cap : 16*P;
-    const size_t per_pool = up(P*48) + 3*up(P*8) + 8*up(P*4) + 2*up(P*16);
-    const size_t rest = 2*up(level_cap*8) + up(isect_cap*8) + up(isect_cap*8) + up(P*4);
+    // a pool's planes; the level kernels also keep a walk record and a flag
+    const size_t per_pool = up(P*48) + 3*up(P*8) + 7*up(P*4) + (queues ? up(P*4) + 2*up(P*16) : 0);
+    const size_t rest = 2*up(level_cap*8) + up(isect_cap*8) + up(isect_cap*8) + (queues ? up(P*4) : 0);
     MLGPU_CUDA(scene->wave.reserve(kWaveCounterBytes + 2*per_pool + rest));
     const int rc = wave_host_counters(scene);
     if (rc) return rc;
@@ -574,9 +581,9 @@ int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32
         int32_t** i[7] = {&p->photon, &p->root, &p->n_int, &p->k_draw, &p->err, &p->step,
                           &p->best_leaf};
         for (int32_t** q : i) *q = reinterpret_cast<int32_t*>(take(P*4));
-        p->overflow_flag = reinterpret_cast<uint32_t*>(take(P*4));
-        p->ray_o = reinterpret_cast<float4*>(take(P*16));
-        p->ray_i = reinterpret_cast<float4*>(take(P*16));
+        p->overflow_flag = queues ? reinterpret_cast<uint32_t*>(take(P*4)) : nullptr;
+        p->ray_o = queues ? reinterpret_cast<float4*>(take(P*16)) : nullptr;
+        p->ray_i = queues ? reinterpret_cast<float4*>(take(P*16)) : nullptr;
     }
     w->pool = pool;
     w->grid = grid > 0 ? grid : scene->wave_grid;
@@ -588,7 +595,7 @@ int wave_buffers(mlgpu_scene* scene, uint32_t pool, int grid, int staged, uint32
     w->slot_leaf_of = scene->dev.slot_leaf;
     w->isect_dist = reinterpret_cast<double*>(take(isect_cap*8));
     w->isect_cap = (uint32_t)isect_cap;
-    w->overflow = reinterpret_cast<uint32_t*>(take(P*4));
+    w->overflow = queues ? reinterpret_cast<uint32_t*>(take(P*4)) : nullptr;
     w->fn_smem_bytes = table_smem_bytes(scene);
     return MLGPU_OK;
 }
@@ -755,7 +762,8 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     // the FP32 forms' double-precision parts are contracted as the compiler
     // sees fit: a second kernel would round them differently
     const bool finish = walk == MLGPU_WALK_STACK && form == MLGPU_TRACER_FP64;
-    const uint32_t want = st->pool_size ? st->pool_size : kWavePool;
+    const uint32_t want = st->pool_size ? st->pool_size
+        : walk == MLGPU_WALK_STACK && !feed ? kWalkPool : kWavePool;
     if (feed) {
         a.sorted = feed->records;
         a.order = nullptr;
@@ -818,7 +826,7 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     // and ties, the overflow walk, resolve and its counters
     const bool stack = w.walk == MLGPU_WALK_STACK;
     const int walk_launches = stack ? 1 : scene->dev.bvh_levels;
-    const int iteration_launches = stack ? 5 : walk_launches + 7;
+    const int iteration_launches = stack ? 2 : walk_launches + 7;
     uint64_t iteration = 0;
     bool more = a.num_photons > pool;   // photons wait for slots
     while (true) {
@@ -846,8 +854,8 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
                     ch.n = 5;
                     const int cls[4] = {MLGPU_KERNEL_INTAKE, MLGPU_KERNEL_WALK,
                                         MLGPU_KERNEL_INTERSECT, MLGPU_KERNEL_RESOLVE};
-                    const int launches[4] = {stack ? 0 : 2, stack ? 3 : walk_launches,
-                                             stack ? 0 : 2, stack ? 2 : 3};
+                    const int launches[4] = {stack ? 0 : 2, stack ? 1 : walk_launches,
+                                             stack ? 0 : 2, stack ? 1 : 3};
                     for (int k = 0; k < 4; k++) { ch.cls[k] = cls[k]; ch.launches[k] = launches[k]; }
                     scene->prof.add(ch);
                 }

@@ -88,11 +88,6 @@ inline int finish_blocks(uint32_t rays) {
     return (int)(need < 148u*kFinishBlocks ? need : 148u*kFinishBlocks);
 }
 
-inline int tree_blocks(uint32_t rays) {
-    const uint32_t need = (rays + 127)/128;
-    return (int)(need < 148u*8u ? need : 148u*8u);
-}
-
 // A lane's walk.
 struct WalkLane {
     float ox, oy, oz;            // origin

@@ -267,6 +267,8 @@ struct WaveCounters {
     unsigned int total;              // active + new photons of this iteration
     unsigned int next;               // survivors written to the next pool
     unsigned int next_inside;        // of them, from its end
+    unsigned int chunks;             // chunks of slots the walk's warps have taken
+    unsigned int blocks;             // blocks of the resolve step that are done
     unsigned int isect_len;          // (slot, leaf) candidates to intersect
     unsigned int overflow_len;       // slots sent to merlict's own walk
     unsigned int level_len[kMaxBvhLevels];   // (slot, node) pairs of each BVH level
@@ -350,8 +352,6 @@ cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* ho
 // recorded between them
 void launch_wave32_hit(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                        cudaStream_t s);
-void launch_wave32_tree(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur, int front,
-                        cudaStream_t s);
 void launch_wave32_resolve(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                            const RayPool& nxt, bool pure, cudaStream_t s);
 cudaError_t launch_wave32_isect_resolve(const TraceArgs& a, const WaveBuffers& w,

@@ -121,6 +121,15 @@ __device__ __forceinline__ int step_kind(const TraceArgs& a, const WaveBuffers& 
                                                                                  : kStepNone;
 }
 
+// The new photons of an iteration, which fill the pool's free slots; a fed
+// propagation admits only those whose records have arrived.
+__device__ __forceinline__ uint32_t new_photons(const TraceArgs& a, const WaveBuffers& w) {
+    const unsigned long long limit = a.fed ? w.counters->avail_snap : a.num_photons;
+    const unsigned long long remaining = limit - w.counters->next_input;
+    const uint32_t room = w.pool - w.counters->active - w.counters->inside;
+    return (uint32_t)(remaining < room ? remaining : room);
+}
+
 // What the level kernels keep of a ray in slot `slot`: its cleared closest
 // hit and, for a BVH walk, its FP32 walk record.
 __device__ __forceinline__ void prepare_levels(const DevScene& sc, const RayPool& p, uint32_t slot,
@@ -244,14 +253,9 @@ wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
         threadIdx.x;
     const uint32_t active = w.counters->active;
     const unsigned long long next_input = w.counters->next_input;
-    // a fed propagation admits only the photons whose records have arrived
-    const unsigned long long limit = a.fed ? w.counters->avail_snap : a.num_photons;
-    const unsigned long long remaining = limit - next_input;
-    const uint32_t inside = w.counters->inside;
-    const uint32_t room = w.pool - active - inside;
-    const uint32_t total = active + (uint32_t)(remaining < room ? remaining : room);
-    const uint32_t chunks = (total + 31)/32, stride = gridDim.x*kWarps;
-    uint32_t chunk = blockIdx.x*kWarps + warp;
+    const uint32_t total = active + new_photons(a, w);
+    const uint32_t chunks = (total + 31)/32;
+    uint32_t chunk = blockIdx.x*kWarps + warp;   // then the next that no warp has
     int taken = 0;               // slots of this chunk given out
     WalkLane l;
     l.walking = false;
@@ -295,29 +299,14 @@ wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
                 }
             }
             taken += take;
-            if (taken == 32) { chunk += stride; taken = 0; }
+            if (taken == 32) {
+                if (lane == 0) chunk = gridDim.x*kWarps + atomicAdd(&w.counters->chunks, 1u);
+                chunk = __shfl_sync(kFull, chunk, 0);
+                taken = 0;
+            }
             __syncwarp();
         }
         groups = visit_nodes(sc, sw, stack, lane, groups, &l);
-    }
-}
-
-// The rays whose hit merlict's own walk of a frame subtree finds: those
-// inside a lens, from the pool's end, and with `front` also new photons
-// (start_node inside a subtree, no BVH, or the frame tree asked for).
-template <int kIsect>
-__global__ void __launch_bounds__(128)
-wave_tree_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, int front) {
-    const uint32_t inside = w.counters->inside;
-    const uint32_t rays = inside + (front ? w.counters->total : 0u);
-    for (uint32_t k = blockIdx.x*blockDim.x + threadIdx.x; k < rays; k += gridDim.x*blockDim.x) {
-        const uint32_t slot = k < inside ? w.pool - 1u - k : k - inside;
-        if (cur.step[slot] != kStepTree) continue;
-        v3 s, d;
-        load_ray(cur, slot, &s, &d);
-        double dist;
-        cur.best_leaf[slot] = closest_hit_tree<kIsect>(a.scene, cur.root[slot], s, d, &dist);
-        cur.best_key[slot] = (unsigned long long)__double_as_longlong(dist);
     }
 }
 
@@ -479,14 +468,14 @@ __device__ __forceinline__ bool resolve_photon(const TraceArgs& a, const double*
                 absorbed = draw() > survival;
             }
         }
+        v3 out = d;              // the new direction in the leaf's frame, if it moves
         if (!hit || absorbed) {
             kind = MLGPU_ABSORPTION_IN_VOID;
         } else {
             const double refl = func_eval_tab(fn_pts, fn_off, table(MLGPU_SURF_OUTER_REFLECTION, MLGPU_SURF_INNER_REFLECTION), lambda, &err);
             if (refl >= draw()) {
                 kind = MLGPU_REFLECTION_ON_SURFACE;
-                s = position(T, is.pos);
-                d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                out = mirror(is.normal, orientation_inverse(T, d));
                 moved = true;
             } else if (!(__ldg(&L->flags) & MLGPU_FLAG_TRANSPARENT)) {
                 kind = MLGPU_ABSORPTION_ON_SURFACE;
@@ -509,8 +498,7 @@ __device__ __forceinline__ bool resolve_photon(const TraceArgs& a, const double*
                 }
                 if (R > draw()) {
                     kind = MLGPU_FRESNEL_REFLECTION_ON_SURFACE;
-                    s = position(T, is.pos);
-                    d = normalized(orientation(T, mirror(is.normal, orientation_inverse(T, d))));
+                    out = mirror(is.normal, inc);
                     moved = true;
                 } else {
                     kind = is.outside ? MLGPU_REFRACTION_TO_INSIDE : MLGPU_REFRACTION_TO_OUTSIDE;
@@ -519,12 +507,15 @@ __device__ __forceinline__ bool resolve_photon(const TraceArgs& a, const double*
                         ? (flags & MLGPU_FLAG_INNER_REFRACTION_DEFAULT) != 0
                         : (flags & MLGPU_FLAG_OUTER_REFRACTION_DEFAULT) != 0;
                     root = (allowed >= 0 && !to_default) ? allowed : 0;
-                    const v3 refr = add(scale(inc, ratio), scale(nrm, ratio*cosI - cosT));
-                    s = position(T, is.pos);
-                    d = normalized(orientation(T, refr));
+                    out = add(scale(inc, ratio), scale(nrm, ratio*cosI - cosT));
                     moved = true;
                 }
             }
+        }
+        if (moved) {
+            // the new ray, whichever way its direction came about
+            s = position(T, is.pos);
+            d = normalized(orientation(T, out));
         }
         if (hist) store_hist(&hist[n_int], is.pos, is.normal, is.dist, is.leaf, kind, is.outside);
         {
@@ -758,36 +749,40 @@ wave_finish_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, in
     }
 }
 
-// 72 registers, seven blocks of 128 per SM: the step waits on its gathers and
-// on chains of double-precision arithmetic, so more warps win over fewer
-// spills (four blocks without spills 4.8 ms per 1e7 photons on the
-// light-field telescope, five to eight blocks 4.5, 4.4, 4.3, 4.3).
-constexpr int kResolveThreads = 128;
-constexpr int kResolveBlocks = 7;
+// The value of avail the next iteration admits photons up to: read once
+// per iteration, so that the intake and its counting agree on it.  avail is
+// raised by kernels of another stream after the records they publish are
+// written, so a fence orders the read before the intake's record reads.
+__device__ __forceinline__ void snapshot_avail(WaveCounters* c) {
+    c->avail_snap = atomicAdd(&c->avail, 0ull);
+    __threadfence();
+}
 
+// One slot of the resolve step, all lanes of the warp: the photon's step,
+// and the photon into the next pool if it goes on.
 template <typename Out, int kIsect>
-__global__ void __launch_bounds__(kResolveThreads, kResolveBlocks)
-wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, const RayPool nxt) {
+__device__ __forceinline__ void resolve_slot(const TraceArgs& a, const WaveBuffers& w,
+                                             const RayPool& cur, const RayPool& nxt,
+                                             const double* fn_pts, const int32_t* fn_off,
+                                             bool valid, uint32_t slot, int lane) {
     const DevScene& sc = a.scene;
-    extern __shared__ double s_fn[];
-    const double* fn_pts;
-    const int32_t* fn_off;
-    stage_tables(sc, w.fn_smem_bytes, s_fn, &fn_pts, &fn_off);
-    const uint32_t total = w.counters->total;
-    const uint32_t index = blockIdx.x*blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const bool valid = index < total + w.counters->inside;
-    const uint32_t slot = index < total ? index : w.pool - 1u - (index - total);
-
     bool survive = false;
     int32_t finished_chunk = -1;   // fed propagation: the chunk of a photon that ends here
     PhotonRay q;
     if (valid) {
         load_photon(cur, slot, &q);
-        survive = resolve_photon<Out, kIsect>(
-            a, fn_pts, fn_off, cur.step[slot], cur.best_leaf[slot],
-            kIsect == kIsectFp64 ? __longlong_as_double((long long)cur.best_key[slot]) : 0.0, &q,
-            [&](v3* s, v3* d) { load_ray(cur, slot, s, d); });
+        const int step = cur.step[slot];
+        int32_t best = kNoLeaf;
+        double dist = 0.0;
+        if (step == kStepTree && w.walk != MLGPU_WALK_LEVELS) {
+            // a ray inside a lens (or without a BVH)
+            best = closest_hit_tree<kIsect>(sc, q.root, q.s, q.d, &dist);
+        } else {
+            best = cur.best_leaf[slot];
+            if (kIsect == kIsectFp64) dist = __longlong_as_double((long long)cur.best_key[slot]);
+        }
+        survive = resolve_photon<Out, kIsect>(a, fn_pts, fn_off, step, best, dist, &q,
+                                              [&](v3* s, v3* d) { load_ray(cur, slot, s, d); });
         if (!survive && a.fed) {
             int32_t c = 0;
             while (c + 1 < a.feed_chunks && (uint64_t)q.photon >= a.feed_start[c + 1]) c++;
@@ -826,6 +821,62 @@ wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, c
             store_photon(nxt, o, q, step);
             if (w.walk == MLGPU_WALK_LEVELS) prepare_levels(sc, nxt, o, q.s, q.d, step);
         }
+    }
+}
+
+// A thread per ray; those inside a lens search their hit first, by merlict's
+// walk of the lens.  96 registers and a few dozen bytes spilled, five blocks
+// of 128 per SM: the step waits on its gathers and on chains of
+// double-precision arithmetic.  1e7 photons of the light-field telescope take
+// 17.65 ms so, and 17.8, 18.0 and 18.1 ms with six to eight blocks.  As three
+// kernels (lens search, resolve, counters) of their own an iteration ended
+// three times: 18.3 ms.
+constexpr int kResolveThreads = 128;
+constexpr int kResolveBlocks = 5;
+
+inline int resolve_blocks(uint32_t pool) {
+    const uint32_t need = (pool + kResolveThreads - 1)/kResolveThreads;
+    return (int)(need < 148u*kResolveBlocks ? need : 148u*kResolveBlocks);
+}
+
+template <typename Out, int kIsect>
+__global__ void __launch_bounds__(kResolveThreads, kResolveBlocks)
+wave_resolve_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur, const RayPool nxt) {
+    const DevScene& sc = a.scene;
+    extern __shared__ double s_fn[];
+    const double* fn_pts;
+    const int32_t* fn_off;
+    stage_tables(sc, w.fn_smem_bytes, s_fn, &fn_pts, &fn_off);
+    const bool levels = w.walk == MLGPU_WALK_LEVELS;
+    const uint32_t fresh = levels ? 0u : new_photons(a, w);
+    const uint32_t front = levels ? w.counters->total : w.counters->active + fresh;
+    const uint32_t rays = front + w.counters->inside;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t first = warp_first(); first < rays; first += gridDim.x*blockDim.x) {
+        const uint32_t index = first + (uint32_t)lane;
+        resolve_slot<Out, kIsect>(a, w, cur, nxt, fn_pts, fn_off, index < rays,
+                                  index < front ? index : w.pool - 1u - (index - front), lane);
+    }
+    if (levels) return;
+    // the last block to end turns the counters over for the next iteration
+    __shared__ bool s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&w.counters->blocks, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x == 0) {
+        WaveCounters* c = w.counters;
+        __threadfence();
+        c->next_input += fresh;
+        c->active = *const_cast<volatile unsigned int*>(&c->next);
+        c->inside = *const_cast<volatile unsigned int*>(&c->next_inside);
+        c->next = 0;
+        c->next_inside = 0;
+        c->chunks = 0;
+        c->blocks = 0;
+        if (a.fed) snapshot_avail(c);
     }
 }
 

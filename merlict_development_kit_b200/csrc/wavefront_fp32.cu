@@ -26,24 +26,19 @@ void launch_wave32_hit(const TraceArgs& a, const WaveBuffers& w, const RayPool& 
         wave_hit_kernel<float, kIsectFp32><<<blocks, kWalkThreads, smem, s>>>(a, w, cur);
 }
 
-void launch_wave32_tree(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur, int front,
-                        cudaStream_t s) {
-    wave_tree_kernel<kIsectFp32><<<tree_blocks(w.pool), 128, 0, s>>>(a, w, cur, front);
-}
-
 void launch_wave32_resolve(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                            const RayPool& nxt, bool pure, cudaStream_t s) {
-    const int resolve_blocks = (int)((w.pool + kResolveThreads - 1)/kResolveThreads);
+    const int blocks = resolve_blocks(w.pool);
     if (pure) {
         if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp32Pure><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<double, kIsectFp32Pure><<<blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
         else
-            wave_resolve_kernel<float, kIsectFp32Pure><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<float, kIsectFp32Pure><<<blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
     } else {
         if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp32><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<double, kIsectFp32><<<blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
         else
-            wave_resolve_kernel<float, kIsectFp32><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<float, kIsectFp32><<<blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
     }
 }
 

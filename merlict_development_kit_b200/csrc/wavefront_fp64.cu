@@ -322,21 +322,11 @@ __global__ void wave_after_intake_kernel(WaveCounters* c, uint32_t pool, uint64_
                                          int fed) {
     const unsigned long long limit = fed ? c->avail_snap : num_photons;
     const unsigned long long remaining = limit - c->next_input;
-    const uint32_t room = pool - c->active - c->inside;
+    const uint32_t room = pool - c->active;
     const uint32_t fresh = (uint32_t)(remaining < room ? remaining : room);
     c->total = c->active + fresh;
     c->next_input += fresh;
     c->next = 0;
-    c->next_inside = 0;
-}
-
-// The value of avail the next iteration admits photons up to: read once
-// here, so that the intake and its counter kernel agree on it.  avail is
-// raised by kernels of another stream after the records they publish are
-// written, so a fence orders the read before the intake's record reads.
-__device__ __forceinline__ void snapshot_avail(WaveCounters* c) {
-    c->avail_snap = atomicAdd(&c->avail, 0ull);
-    __threadfence();
 }
 
 __global__ void wave_after_resolve_kernel(WaveCounters* c, int fed) {
@@ -344,7 +334,6 @@ __global__ void wave_after_resolve_kernel(WaveCounters* c, int fed) {
         if (fed) snapshot_avail(c);
         c->overflow_total += c->overflow_len;
         c->active = c->next;
-        c->inside = c->next_inside;
         c->isect_len = 0;
         c->overflow_len = 0;
     }
@@ -390,13 +379,11 @@ cudaError_t launch_wave_counters_to_host(const WaveCounters* c, WaveCounters* ho
 cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, const RayPool& cur,
                                   const RayPool& nxt, int form, cudaStream_t s, cudaEvent_t* ev) {
     const int slot_blocks = (int)((w.pool + 255)/256);
-    const int resolve_blocks = (int)((w.pool + kResolveThreads - 1)/kResolveThreads);
+    const int blocks_of_resolve = resolve_blocks(w.pool);
     if (ev) cudaEventRecord(ev[0], s);
     if (w.walk == MLGPU_WALK_STACK) {
         // intake, walk and intersections in one kernel
         if (ev) cudaEventRecord(ev[1], s);
-        const int front = a.start_node != 0 || a.scene.surf_levels == 0 ||
-            a.traversal == MLGPU_TRAVERSAL_FRAME_TREE;
         if (form == MLGPU_TRACER_FP64) {
             const int blocks = walk_blocks(w.pool);
             const size_t smem = closest_hit_smem(a.scene.surf_levels);
@@ -407,22 +394,16 @@ cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, cons
         } else {
             launch_wave32_hit(a, w, cur, s);
         }
-        wave_after_intake_kernel<<<1, 1, 0, s>>>(w.counters, w.pool, a.num_photons, a.fed);
-        if (form == MLGPU_TRACER_FP64)
-            wave_tree_kernel<kIsectFp64><<<tree_blocks(w.pool), 128, 0, s>>>(a, w, cur, front);
-        else
-            launch_wave32_tree(a, w, cur, front, s);
         if (ev) cudaEventRecord(ev[2], s);
         if (ev) cudaEventRecord(ev[3], s);
         if (form == MLGPU_TRACER_FP64) {
             if (a.out_dtype == MLGPU_F64)
-                wave_resolve_kernel<double, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+                wave_resolve_kernel<double, kIsectFp64><<<blocks_of_resolve, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
             else
-                wave_resolve_kernel<float, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+                wave_resolve_kernel<float, kIsectFp64><<<blocks_of_resolve, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
         } else {
             launch_wave32_resolve(a, w, cur, nxt, false, s);
         }
-        wave_after_resolve_kernel<<<1, 64, 0, s>>>(w.counters, a.fed);
         if (ev) cudaEventRecord(ev[4], s);
         return cudaGetLastError();
     }
@@ -444,9 +425,9 @@ cudaError_t launch_wave_iteration(const TraceArgs& a, const WaveBuffers& w, cons
         if (ev) cudaEventRecord(ev[3], s);
         wave_overflow_kernel<<<148, 128, 0, s>>>(a, w, cur);
         if (a.out_dtype == MLGPU_F64)
-            wave_resolve_kernel<double, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<double, kIsectFp64><<<blocks_of_resolve, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
         else
-            wave_resolve_kernel<float, kIsectFp64><<<resolve_blocks, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
+            wave_resolve_kernel<float, kIsectFp64><<<blocks_of_resolve, kResolveThreads, w.fn_smem_bytes, s>>>(a, w, cur, nxt);
     } else {
         const cudaError_t e = launch_wave32_isect_resolve(a, w, cur, nxt,
                                                           form == MLGPU_TRACER_FP32_PURE, s,
