@@ -212,9 +212,77 @@ __device__ __forceinline__ void img_store8(uint8_t* img, uint32_t rows, uint32_t
     q.z = pack_bf16x2(v[4], v[5]); q.w = pack_bf16x2(v[6], v[7]);
     *reinterpret_cast<uint4*>(img + img_off(rows, r, k)) = q;
 }
-__device__ __forceinline__ void img_store1(uint8_t* img, uint32_t rows, uint32_t r, uint32_t k,
-                                           float v) {
-    *reinterpret_cast<__nv_bfloat16*>(img + img_off(rows, r, k)) = __float2bfloat16_rn(v);
+// Stores 16 consecutive k values (k a multiple of 16) of row r of an image:
+// the two 16-byte chunks of a 32-byte sector, in the order the swizzle puts
+// them, in one store.
+__device__ __forceinline__ void img_store16(uint8_t* img, uint32_t rows, uint32_t r, uint32_t k,
+                                            const uint32_t* w) {
+    uint8_t* p = img + (img_off(rows, r, k) & ~(uint64_t)31);
+    const bool odd = (r & 1u) != 0;
+    const uint4 a = make_uint4(odd ? w[4] : w[0], odd ? w[5] : w[1], odd ? w[6] : w[2],
+                               odd ? w[7] : w[3]);
+    const uint4 b = make_uint4(odd ? w[0] : w[4], odd ? w[1] : w[5], odd ? w[2] : w[6],
+                               odd ? w[3] : w[7]);
+    if ((reinterpret_cast<uintptr_t>(img) & 31u) == 0) {
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                     :: "l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y),
+                        "r"(b.z), "r"(b.w)
+                     : "memory");
+    } else {   // a caller's workspace on a 16-byte boundary
+        reinterpret_cast<uint4*>(p)[0] = a;
+        reinterpret_cast<uint4*>(p)[1] = b;
+    }
+}
+
+// A warp's 32 x 32 block (lane: row, v: columns) to the image of a matrix
+// and, if img_t is not null, of its transpose: rows row0 + lane, columns nb
+// + j.  The transpose goes through 32 x 17 words of shared memory, so that
+// both images are written in whole 32-byte sectors: written two bytes a lane
+// the transposes took two thirds of a training step.
+constexpr int kTileWords = 32*17;
+__device__ __forceinline__ void store_block(uint8_t* img, uint32_t img_rows, uint8_t* img_t,
+                                            uint32_t img_t_rows, uint32_t row0, uint32_t nb,
+                                            const float* v, uint32_t* tile, int lane) {
+    uint32_t w[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) w[j] = pack_bf16x2(v[2*j], v[2*j + 1]);
+    if (img) {
+        img_store16(img, img_rows, row0 + (uint32_t)lane, nb, w);
+        img_store16(img, img_rows, row0 + (uint32_t)lane, nb + 16, w + 8);
+    }
+    if (img_t) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 16; j++) tile[lane*17 + j] = w[j];
+        __syncwarp();
+        // this lane: columns 2 c and 2 c + 1 of rows 16 h .. 16 h + 15
+        const int c = lane & 15, h = lane >> 4;
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint32_t a = tile[(16*h + 2*k)*17 + c], b = tile[(16*h + 2*k + 1)*17 + c];
+            lo[k] = __byte_perm(a, b, 0x5410);
+            hi[k] = __byte_perm(a, b, 0x7632);
+        }
+        const uint32_t r = nb + 2u*(uint32_t)c, k0 = row0 + 16u*(uint32_t)h;
+        img_store16(img_t, img_t_rows, r, k0, lo);
+        img_store16(img_t, img_t_rows, r + 1, k0, hi);
+    }
+}
+
+// Column sums of a warp's 32 x 32 block: lane j gets column j's (v is used
+// up).  Halving the columns kept at each step takes 31 exchanges.
+__device__ __forceinline__ float column_sum(float* v, int lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int j = 0; j < o; j++) {
+            const float keep = up ? v[j + o] : v[j], give = up ? v[j] : v[j + o];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0];
 }
 
 // ---- the GEMM ------------------------------------------------------------------
@@ -230,7 +298,8 @@ struct GemmArgs {
     float* out; uint32_t ld; uint64_t split_stride; uint32_t n_store;   // FP32 C
     uint8_t* img; uint32_t img_rows;       // image of the result (rows = M, K = N)
     uint8_t* img_t; uint32_t img_t_rows;   // image of its transpose (rows = N, K = M)
-    float* z; uint32_t z_ld;               // pre-activations: written (SiLU) or read (dSiLU)
+    float* z;                              // pre-activations (kH columns), written (SiLU) or read
+                                           // (dSiLU), in blocks of 32 x 32: see z_block
     float* col_sum;                        // [N] column sums of the result (dSiLU)
 };
 
@@ -243,7 +312,31 @@ __host__ __device__ constexpr uint32_t tmem_cols() {
     return kN <= 32 ? 32u : kN <= 64 ? 64u : kN <= 128 ? 128u : 256u;
 }
 
-template <int kN, int kEpi>
+// The epilogue of one 32-column slice of row `row`: C in FP32.
+__device__ __forceinline__ void epilogue_f32(const GemmArgs& g, uint32_t row, uint32_t nb,
+                                             uint32_t split, float* v) {
+    if (g.bias) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] += (nb + j < g.bias_n) ? __ldg(g.bias + nb + j) : 0.0f;
+    }
+    float* o = g.out + (uint64_t)split*g.split_stride + (uint64_t)row*g.ld + nb;
+    if (nb + 32 <= g.n_store && (g.ld & 3u) == 0) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    } else {
+        for (int j = 0; j < 32; j++) if (nb + j < g.n_store) o[j] = v[j];
+    }
+}
+
+// The pre-activations of rows 32 i .. 32 i + 31 and columns nb .. nb + 31,
+// 1,024 floats: four columns of a lane's row after one another, then the next
+// lane's, so that a warp reads and writes them in whole lines.
+__device__ __forceinline__ float4* z_block(float* z, uint32_t row0, uint32_t nb, int lane) {
+    return reinterpret_cast<float4*>(z + ((uint64_t)(row0 >> 5)*(kH/32) + (nb >> 5))*1024) + lane;
+}
+
+template <int kN>
 __global__ void __launch_bounds__(kThreads, 1)
 umma_gemm_kernel(const GemmArgs g) {
     extern __shared__ uint8_t smem_raw[];
@@ -329,61 +422,7 @@ umma_gemm_kernel(const GemmArgs g) {
         for (uint32_t c0 = 0; ok && c0 < (uint32_t)kN; c0 += 32) {
             float v[32];
             tmem_ld32(taddr + c0, v);
-            const uint32_t nb = n0 + c0;
-            if (kEpi == kEpiF32) {
-                if (g.bias) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] += (nb + j < g.bias_n) ? __ldg(g.bias + nb + j) : 0.0f;
-                }
-                float* o = g.out + (uint64_t)blockIdx.z*g.split_stride + (uint64_t)row*g.ld + nb;
-                if (nb + 32 <= g.n_store && (g.ld & 3u) == 0) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4)
-                        *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                } else {
-                    for (int j = 0; j < 32; j++) if (nb + j < g.n_store) o[j] = v[j];
-                }
-            } else if (kEpi == kEpiSilu) {
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    const float zz = v[j] + __ldg(g.bias + nb + j);
-                    if (g.z) g.z[(uint64_t)row*g.z_ld + nb + j] = zz;
-                    v[j] = silu(zz);
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j += 8) img_store8(g.img, g.img_rows, row, nb + j, v + j);
-                if (g.img_t) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) img_store1(g.img_t, g.img_t_rows, nb + j, row, v[j]);
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; j++)
-                    v[j] *= dsilu(g.z[(uint64_t)row*g.z_ld + nb + j]);
-                if (g.img) {
-#pragma unroll
-                    for (int j = 0; j < 32; j += 8) img_store8(g.img, g.img_rows, row, nb + j, v + j);
-                }
-                if (g.img_t) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) img_store1(g.img_t, g.img_t_rows, nb + j, row, v[j]);
-                }
-                if (g.out) {
-                    float* o = g.out + (uint64_t)row*g.ld + nb;
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4)
-                        *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                }
-                if (g.col_sum) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        float t = v[j];
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                        if (lane == 0) atomicAdd(g.col_sum + nb + j, t);
-                    }
-                }
-            }
+            epilogue_f32(g, row, n0 + c0, blockIdx.z, v);
         }
     }
     tc_fence_before();
@@ -409,63 +448,38 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
 }
 
-// The epilogue of one 32-column slice of row `row` (shared by both GEMMs).
+// The epilogue of one 32-column slice of the rows row0 + lane; `tile`: the
+// warp's shared memory for transposes.  Returns the column sum of the lane's
+// column with kEpiDSilu.
 template <int kEpi>
-__device__ __forceinline__ void epilogue32(const GemmArgs& g, uint32_t row, uint32_t nb,
-                                           uint32_t split, float* v, int lane) {
+__device__ __forceinline__ float epilogue32(const GemmArgs& g, uint32_t row0, uint32_t nb, float* v,
+                                            uint32_t* tile, int lane) {
     if (kEpi == kEpiF32) {
-        if (g.bias) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] += (nb + j < g.bias_n) ? __ldg(g.bias + nb + j) : 0.0f;
-        }
-        float* o = g.out + (uint64_t)split*g.split_stride + (uint64_t)row*g.ld + nb;
-        if (nb + 32 <= g.n_store && (g.ld & 3u) == 0) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        } else {
-            for (int j = 0; j < 32; j++) if (nb + j < g.n_store) o[j] = v[j];
-        }
-    } else if (kEpi == kEpiSilu) {
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            const float zz = v[j] + __ldg(g.bias + nb + j);
-            if (g.z) g.z[(uint64_t)row*g.z_ld + nb + j] = zz;
-            v[j] = silu(zz);
-        }
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) img_store8(g.img, g.img_rows, row, nb + j, v + j);
-        if (g.img_t) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) img_store1(g.img_t, g.img_t_rows, nb + j, row, v[j]);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] *= dsilu(g.z[(uint64_t)row*g.z_ld + nb + j]);
-        if (g.img) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) img_store8(g.img, g.img_rows, row, nb + j, v + j);
-        }
-        if (g.img_t) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) img_store1(g.img_t, g.img_t_rows, nb + j, row, v[j]);
-        }
-        if (g.out) {
-            float* o = g.out + (uint64_t)row*g.ld + nb;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        }
-        if (g.col_sum) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-                float t = v[j];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                if (lane == 0) atomicAdd(g.col_sum + nb + j, t);
-            }
-        }
+        epilogue_f32(g, row0 + (uint32_t)lane, nb, 0, v);
+        return 0.0f;
     }
+    if (kEpi == kEpiSilu) {
+        float4* z = g.z ? z_block(g.z, row0, nb, lane) : nullptr;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+#pragma unroll
+            for (int i = j; i < j + 4; i++) v[i] += __ldg(g.bias + nb + i);
+            if (z) z[8*j] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+#pragma unroll
+            for (int i = j; i < j + 4; i++) v[i] = silu(v[i]);
+        }
+        store_block(g.img, g.img_rows, g.img_t, g.img_t_rows, row0, nb, v, tile, lane);
+        return 0.0f;
+    }
+    const float4* z = z_block(g.z, row0, nb, lane);
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        const float4 zz = z[8*j];
+        v[j] *= dsilu(zz.x); v[j + 1] *= dsilu(zz.y);
+        v[j + 2] *= dsilu(zz.z); v[j + 3] *= dsilu(zz.w);
+    }
+    store_block(g.img, g.img_rows, g.img_t, g.img_t_rows, row0, nb, v, tile, lane);
+    return column_sum(v, lane);
 }
 
 // ---- the persistent, weight-resident GEMM ------------------------------------------
@@ -480,9 +494,10 @@ __device__ __forceinline__ void epilogue32(const GemmArgs& g, uint32_t row, uint
 
 constexpr int kARing = 4;
 
-template <int kN, int kKChunks>
+template <int kN, int kKChunks, int kEpi>
 __host__ __device__ constexpr uint32_t pers_smem_bytes() {
-    return (uint32_t)kKChunks*(uint32_t)kN*128u + kARing*16384u + 1024u + 256u;
+    return (uint32_t)kKChunks*(uint32_t)kN*128u + kARing*16384u + 1024u + 256u +
+        (kEpi == kEpiF32 ? 0u : 8u*(uint32_t)kTileWords*4u);
 }
 
 template <int kN, int kKChunks, int kEpi>
@@ -585,22 +600,35 @@ umma_persistent_kernel(const GemmArgs g, uint32_t num_tiles) {
         // take the even 32-column slices, warps 6..9 the odd ones
         const uint32_t q = (uint32_t)warp & 3u;
         const uint32_t half = (uint32_t)(warp - 2) >> 2;
+        uint32_t* tile_words = reinterpret_cast<uint32_t*>(smem + kBBytes + kARing*16384u + 256u) +
+            (warp - 2)*kTileWords;
+        constexpr int kSlices = (kN + 63)/64;
+        float sums[kSlices];               // of this warp's columns over its tiles
+#pragma unroll
+        for (int k = 0; k < kSlices; k++) sums[k] = 0.0f;
         uint32_t t = 0;
         for (uint32_t tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, t++) {
             const uint32_t acc = t & 1u;
             const bool ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (t >> 1) & 1));
             tc_fence_after();
             if (!ok) { s_failed = 1; break; }
-            const uint32_t row = tile*128u + q*32u + (uint32_t)lane;
             const uint32_t taddr = tmem + acc*kCols + ((q*32u) << 16);
-            for (uint32_t c0 = half*32u; c0 < (uint32_t)kN; c0 += 64) {
+#pragma unroll
+            for (int k = 0; k < kSlices; k++) {
+                const uint32_t c0 = half*32u + 64u*(uint32_t)k;
+                if (c0 >= (uint32_t)kN) break;
                 float v[32];
                 tmem_ld32(taddr + c0, v);
-                epilogue32<kEpi>(g, row, c0, 0, v, lane);
+                sums[k] += epilogue32<kEpi>(g, tile*128u + q*32u, c0, v, tile_words, lane);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
+        }
+        if (kEpi == kEpiDSilu && g.col_sum) {
+#pragma unroll
+            for (int k = 0; k < kSlices; k++)
+                atomicAdd(g.col_sum + half*32u + 64u*(uint32_t)k + (uint32_t)lane, sums[k]);
         }
     }
     tc_fence_before();
@@ -636,7 +664,7 @@ int sm_count() {
 // C = A W^T with W (N x 64 kKChunks) resident: m rows (a multiple of 128).
 template <int kN, int kKChunks, int kEpi>
 cudaError_t launch_persistent(const GemmArgs& g, uint32_t m, cudaStream_t s) {
-    constexpr uint32_t smem = pers_smem_bytes<kN, kKChunks>();
+    constexpr uint32_t smem = pers_smem_bytes<kN, kKChunks, kEpi>();
     static bool attr = false;
     if (!attr) {
         const cudaError_t e = cudaFuncSetAttribute(umma_persistent_kernel<kN, kKChunks, kEpi>,
@@ -652,19 +680,19 @@ cudaError_t launch_persistent(const GemmArgs& g, uint32_t m, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int kN, int kEpi>
+template <int kN>
 cudaError_t launch_gemm(const GemmArgs& g, uint32_t m, uint32_t n, uint32_t splits, cudaStream_t s) {
     constexpr uint32_t smem = gemm_smem_bytes<kN>();
     static bool attr = false;
     if (!attr) {
-        const cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<kN, kEpi>,
+        const cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<kN>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)smem);
         if (e != cudaSuccess) return e;
         attr = true;
     }
     const dim3 grid(m/128u, n/(uint32_t)kN, splits);
-    umma_gemm_kernel<kN, kEpi><<<grid, kThreads, smem, s>>>(g);
+    umma_gemm_kernel<kN><<<grid, kThreads, smem, s>>>(g);
     return cudaGetLastError();
 }
 
@@ -719,37 +747,50 @@ __global__ void pack_weights_kernel(const float* __restrict__ p, uint8_t* __rest
 // inputs themselves, then sin(pi 2^l x_j) and cos(pi 2^l x_j) for j = 0..4
 // and l = 0..kFreq-1 (feature 5 + 2 (kFreq j + l) + c), then zeros.  The
 // argument 2^l x_j (a product by a power of two) is exact in FP32 and
-// sincospif reduces it exactly.
-__device__ __forceinline__ float encoded(const float* xi, int f) {
-    if (f < kIn) return xi[f];
-    const int g = f - kIn;
-    if (g >= 2*kFreq*kIn) return 0.0f;
-    const int j = g/(2*kFreq), l = (g % (2*kFreq)) >> 1;
-    float sn, cs;
-    sincospif(__fmul_rn(xi[j], (float)(1 << l)), &sn, &cs);
-    return (g & 1) ? cs : sn;
+// sincospif reduces it exactly.  A warp per 32 rows and 32 features writes
+// them as a tile image (rows = batch, K = kEnc) and, when training, its
+// transpose's image.
+constexpr int kEncodeWarps = 8;
+
+template <int kSlice>
+__device__ __forceinline__ void encode_slice(const float* xi, float* v) {
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+        const int f = 32*kSlice + k, g = f - kIn;
+        if (f < kIn) {
+            v[k] = xi[f < kIn ? f : 0];
+        } else if (g >= 2*kFreq*kIn) {
+            v[k] = 0.0f;
+        } else if (!(g & 1) || k == 0) {
+            // a sine, and the cosine after it
+            const int j = g/(2*kFreq), l = (g % (2*kFreq)) >> 1;
+            float sn, cs;
+            sincospif(__fmul_rn(xi[j], (float)(1 << l)), &sn, &cs);
+            v[k] = (g & 1) ? cs : sn;
+            if (!(g & 1) && k + 1 < 32) v[k + 1] = cs;
+        }
+    }
 }
 
-// One thread per (row, 8 features): the encoded inputs as a tile image
-// (rows = batch, K = kEnc) and, when training, its transpose's image.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32*kEncodeWarps)
 encode_kernel(const float* __restrict__ x, uint32_t batch, uint8_t* __restrict__ img,
               uint8_t* __restrict__ img_t) {
-    const uint64_t t = blockIdx.x*(uint64_t)blockDim.x + threadIdx.x;
-    const uint32_t row = (uint32_t)(t/(kEnc/8));
-    const int f0 = (int)(t % (kEnc/8))*8;
-    if (row >= batch) return;
+    __shared__ uint32_t s_tile[kEncodeWarps][kTileWords];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t job = blockIdx.x*kEncodeWarps + (uint32_t)warp;
+    const uint32_t row0 = (job >> 2)*32u, slice = job & 3u;
+    if (row0 >= batch) return;
     float xi[kIn];
 #pragma unroll
-    for (int j = 0; j < kIn; j++) xi[j] = __ldg(x + (uint64_t)row*kInLd + j);
-    float v[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = encoded(xi, f0 + k);
-    img_store8(img, batch, row, (uint32_t)f0, v);
-    if (img_t) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) img_store1(img_t, kEnc, (uint32_t)(f0 + k), row, v[k]);
+    for (int j = 0; j < kIn; j++) xi[j] = __ldg(x + (uint64_t)(row0 + lane)*kInLd + j);
+    float v[32];
+    switch (slice) {
+    case 0: encode_slice<0>(xi, v); break;
+    case 1: encode_slice<1>(xi, v); break;
+    case 2: encode_slice<2>(xi, v); break;
+    default: encode_slice<3>(xi, v); break;
     }
+    store_block(img, batch, img_t, kEnc, row0, 32u*slice, v, s_tile[warp], lane);
 }
 
 // ---- the fused inference forward ----------------------------------------------------
@@ -826,7 +867,7 @@ struct StepIter {
 };
 
 // Encodes features [64 p + 16 h, + 16) of row r of a tile (inputs xi) into
-// chunk p of the activation image: the values of encoded(), one sincospif
+// chunk p of the activation image: the values of the fixed encoding, one sincospif
 // per (input, octave) for its sine and cosine features.  f0 is the same
 // for the whole warp, so the branches do not diverge.
 __device__ __forceinline__ void encode_part(uint8_t* act, uint32_t r, uint32_t p, uint32_t h,
@@ -1082,25 +1123,30 @@ fused_forward_kernel(const float* __restrict__ p, const uint8_t* __restrict__ im
 // The loss of one photon and its gradient with respect to the 73 outputs
 // (scaled by 1/batch).  Outputs y: reach logit, then per component k:
 // weight logit, 4 means, 4 log-sigmas (clamped to [-9, 3]).
-__device__ float photon_loss(const float* y, const float* t, bool reached, float* dy) {
+__device__ __forceinline__ float photon_loss(const float* y, const float* t, bool reached, float* dy) {
     const float l = y[0];
     const float sig = 1.0f/(1.0f + __expf(-l));
     // softplus(l) - r l, computed stably
     float loss = fmaxf(l, 0.0f) + log1pf(__expf(-fabsf(l))) - (reached ? l : 0.0f);
     dy[0] = sig - (reached ? 1.0f : 0.0f);
+#pragma unroll
     for (int j = 1; j < kOut; j++) dy[j] = 0.0f;
     if (!reached) return loss;
     constexpr int K = MLGPU_SG_COMPONENTS, D = MLGPU_SG_DIMS;
     float amax = -INFINITY;
+#pragma unroll
     for (int k = 0; k < K; k++) amax = fmaxf(amax, y[1 + 9*k]);
     float asum = 0.0f;
+#pragma unroll
     for (int k = 0; k < K; k++) asum += __expf(y[1 + 9*k] - amax);
     const float log_norm = amax + __logf(asum);
     float ell[K];
     float lmax = -INFINITY;
+#pragma unroll
     for (int k = 0; k < K; k++) {
         const float* c = y + 1 + 9*k;
         float e = c[0] - log_norm;
+#pragma unroll
         for (int d = 0; d < D; d++) {
             const float ls = fminf(fmaxf(c[5 + d], -9.0f), 3.0f);
             const float u = (t[d] - c[1 + d])*__expf(-ls);
@@ -1110,14 +1156,17 @@ __device__ float photon_loss(const float* y, const float* t, bool reached, float
         lmax = fmaxf(lmax, e);
     }
     float esum = 0.0f;
+#pragma unroll
     for (int k = 0; k < K; k++) esum += __expf(ell[k] - lmax);
     loss += -(lmax + __logf(esum));
+#pragma unroll
     for (int k = 0; k < K; k++) {
         const float* c = y + 1 + 9*k;
         float* dc = dy + 1 + 9*k;
         const float gam = __expf(ell[k] - lmax)/esum;
         const float pi = __expf(c[0] - log_norm);
         dc[0] = pi - gam;
+#pragma unroll
         for (int d = 0; d < D; d++) {
             const float raw = c[5 + d];
             const float ls = fminf(fmaxf(raw, -9.0f), 3.0f);
@@ -1131,38 +1180,49 @@ __device__ float photon_loss(const float* y, const float* t, bool reached, float
 }
 
 // One thread per photon: loss, dY images (rows = batch, K = 128) and
-// (rows = 128, K = batch), output-bias gradient, loss sum.
-__global__ void __launch_bounds__(256)
+// (rows = 128, K = batch), output-bias gradient, loss sum.  The photon's
+// outputs and their gradients stay in registers; a warp's photons go to the
+// images in blocks of 32 columns, and the bias gradient to device memory as
+// one addition per block and column (an addition per warp and column, through
+// local memory, took 141 us per 65,536 photons).
+constexpr int kLossThreads = 128;
+
+__global__ void __launch_bounds__(kLossThreads)
 loss_kernel(const float* __restrict__ y, const float* __restrict__ targets,
             const uint8_t* __restrict__ reached, uint32_t batch, uint8_t* __restrict__ dy_img,
             uint8_t* __restrict__ dyt_img, float* __restrict__ grad_b4, float* __restrict__ loss_sum) {
-    const uint32_t row = blockIdx.x*blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    float dy[kOutK];
-    float loss = 0.0f;
-    if (row < batch) {
-        float yy[kOut], t[4];
-        for (int j = 0; j < kOut; j++) yy[j] = y[(uint64_t)row*kOutPad + j];
-        for (int d = 0; d < 4; d++) t[d] = targets[(uint64_t)row*4 + d];
-        loss = photon_loss(yy, t, reached[row] != 0, dy);
-        const float inv_b = 1.0f/(float)batch;
-        loss *= inv_b;
-        for (int j = 0; j < kOut; j++) dy[j] *= inv_b;
-    } else {
-        for (int j = 0; j < kOut; j++) dy[j] = 0.0f;
+    __shared__ uint32_t s_tile[kLossThreads/32][kTileWords];
+    __shared__ float s_sum[kOutK + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int j = threadIdx.x; j <= kOutK; j += kLossThreads) s_sum[j] = 0.0f;
+    __syncthreads();
+    const uint32_t row = blockIdx.x*kLossThreads + threadIdx.x;   // batch: a multiple of 128
+    float dy[kOut];
+    float yy[kOut + 3];
+    const float4* y4 = reinterpret_cast<const float4*>(y + (uint64_t)row*kOutPad);
+#pragma unroll
+    for (int j = 0; j < (kOut + 3)/4; j++) {
+        const float4 q = __ldg(y4 + j);
+        yy[4*j] = q.x; yy[4*j + 1] = q.y; yy[4*j + 2] = q.z; yy[4*j + 3] = q.w;
     }
-    for (int j = kOut; j < kOutK; j++) dy[j] = 0.0f;
-    if (row < batch) {
-        for (int j = 0; j < kOutK; j += 8) img_store8(dy_img, batch, row, j, dy + j);
-        for (int j = 0; j < kOutK; j++) img_store1(dyt_img, kOutK, j, row, dy[j]);
-    }
-    for (int j = 0; j < kOut; j++) {
-        float s = dy[j];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) atomicAdd(grad_b4 + j, s);
+    const float t[4] = {targets[(uint64_t)row*4], targets[(uint64_t)row*4 + 1],
+                        targets[(uint64_t)row*4 + 2], targets[(uint64_t)row*4 + 3]};
+    const float inv_b = 1.0f/(float)batch;
+    float loss = photon_loss(yy, t, reached[row] != 0, dy)*inv_b;
+#pragma unroll
+    for (int s = 0; s < kOutK/32; s++) {
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+            v[j] = 32*s + j < kOut ? dy[32*s + j < kOut ? 32*s + j : 0]*inv_b : 0.0f;
+        store_block(dy_img, batch, dyt_img, kOutK, row & ~31u, 32u*s, v, s_tile[warp], lane);
+        if (32*s < kOut) atomicAdd(&s_sum[32*s + lane], column_sum(v, lane));
     }
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if (lane == 0) atomicAdd(loss_sum, loss);
+    if (lane == 0) atomicAdd(&s_sum[kOutK], loss);
+    __syncthreads();
+    if (threadIdx.x < kOut) atomicAdd(grad_b4 + threadIdx.x, s_sum[threadIdx.x]);
+    if (threadIdx.x == kOut) atomicAdd(loss_sum, s_sum[kOutK]);
 }
 
 // Sums the split-K partials of a weight gradient into the gradient buffer
@@ -1172,6 +1232,7 @@ __global__ void reduce_dw_kernel(const float* __restrict__ ws, uint32_t splits, 
     const uint32_t n = out_rows*cols;
     for (uint32_t i = blockIdx.x*blockDim.x + threadIdx.x; i < n; i += gridDim.x*blockDim.x) {
         float s = 0.0f;
+#pragma unroll 16
         for (uint32_t k = 0; k < splits; k++) s += ws[k*stride + i];
         grad[i] = s;
     }
@@ -1344,7 +1405,7 @@ GemmArgs gemm_args(const uint8_t* a, uint32_t a_rows, const uint8_t* b, uint32_t
 // The forward pass (training: also transposed images and pre-activations).
 cudaError_t forward(const float* p, const uint8_t* img, const float* x, uint32_t batch,
                     const Work& w, float* y, bool training, cudaStream_t s) {
-    encode_kernel<<<(uint32_t)(((uint64_t)batch*(kEnc/8) + 255)/256), 256, 0, s>>>(
+    encode_kernel<<<(batch/32u*4u + kEncodeWarps - 1)/kEncodeWarps, 32*kEncodeWarps, 0, s>>>(
         x, batch, w.enc_img, training ? w.enc_imgt : nullptr);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
@@ -1352,7 +1413,7 @@ cudaError_t forward(const float* p, const uint8_t* img, const float* x, uint32_t
         g.bias = p + kB0; g.bias_n = kH;
         g.img = w.h_img[0]; g.img_rows = batch;
         g.img_t = training ? w.h_imgt[0] : nullptr; g.img_t_rows = kH;
-        g.z = training ? w.z[0] : nullptr; g.z_ld = kH;
+        g.z = training ? w.z[0] : nullptr;
         e = launch_persistent<256, kEnc/64, kEpiSilu>(g, batch, s);
     }
     for (int l = 1; l <= 3 && e == cudaSuccess; l++) {
@@ -1360,7 +1421,7 @@ cudaError_t forward(const float* p, const uint8_t* img, const float* x, uint32_t
         g.bias = p + b_off(l); g.bias_n = kH;
         g.img = w.h_img[l]; g.img_rows = batch;
         g.img_t = training ? w.h_imgt[l] : nullptr; g.img_t_rows = kH;
-        g.z = training ? w.z[l] : nullptr; g.z_ld = kH;
+        g.z = training ? w.z[l] : nullptr;
         e = launch_persistent<256, 4, kEpiSilu>(g, batch, s);
     }
     if (e == cudaSuccess) {
@@ -1398,7 +1459,7 @@ cudaError_t train_step(float* p, uint8_t* img, float* m, float* v, const float* 
     if (e == cudaSuccess) e = cudaMemsetAsync(w.loss, 0, 4, s);
     if (e == cudaSuccess) e = forward(p, img, x, batch, w, w.y, true, s);
     if (e != cudaSuccess) return e;
-    loss_kernel<<<(batch + 255)/256, 256, 0, s>>>(w.y, targets, reached, batch, w.dy_img,
+    loss_kernel<<<batch/kLossThreads, kLossThreads, 0, s>>>(w.y, targets, reached, batch, w.dy_img,
                                                    w.dyt_img, w.grads + kB4, w.loss);
     e = cudaGetLastError();
     const uint32_t kchunks = batch/64;
@@ -1409,16 +1470,16 @@ cudaError_t train_step(float* p, uint8_t* img, float* m, float* v, const float* 
     if (e == cudaSuccess) {
         GemmArgs g = gemm_args(w.dyt_img, kOutK, w.h_imgt[3], kH, kchunks/splits);
         g.out = w.ws; g.ld = kH; g.split_stride = ws_stride; g.n_store = kH;
-        e = launch_gemm<256, kEpiF32>(g, kOutK, kH, splits, s);
+        e = launch_gemm<256>(g, kOutK, kH, splits, s);
     }
     if (e == cudaSuccess) {
-        reduce_dw_kernel<<<148, 256, 0, s>>>(w.ws, splits, ws_stride, kOut, kH, w.grads + kW4);
+        reduce_dw_kernel<<<(kOut*kH + 255)/256, 256, 0, s>>>(w.ws, splits, ws_stride, kOut, kH, w.grads + kW4);
         e = cudaGetLastError();
     }
     int cur = 0;
     if (e == cudaSuccess) {
         GemmArgs g = gemm_args(w.dy_img, batch, img + kImgW4TOff, kH, kOutK/64);
-        g.z = w.z[3]; g.z_ld = kH;
+        g.z = w.z[3];
         g.img = w.dz_img[cur]; g.img_rows = batch;
         g.img_t = w.dz_imgt[cur]; g.img_t_rows = kH;
         g.col_sum = w.grads + kB3;
@@ -1428,13 +1489,13 @@ cudaError_t train_step(float* p, uint8_t* img, float* m, float* v, const float* 
     for (int l = 3; l >= 1 && e == cudaSuccess; l--) {
         GemmArgs g = gemm_args(w.dz_imgt[cur], kH, w.h_imgt[l - 1], kH, kchunks/splits);
         g.out = w.ws; g.ld = kH; g.split_stride = ws_stride; g.n_store = kH;
-        e = launch_gemm<256, kEpiF32>(g, kH, kH, splits, s);
+        e = launch_gemm<256>(g, kH, kH, splits, s);
         if (e != cudaSuccess) break;
-        reduce_dw_kernel<<<148, 256, 0, s>>>(w.ws, splits, ws_stride, kH, kH, w.grads + w_off(l));
+        reduce_dw_kernel<<<(kH*kH + 255)/256, 256, 0, s>>>(w.ws, splits, ws_stride, kH, kH, w.grads + w_off(l));
         e = cudaGetLastError();
         if (e != cudaSuccess) break;
         GemmArgs d = gemm_args(w.dz_img[cur], batch, img + img_wt(l), kH, kH/64);
-        d.z = w.z[l - 1]; d.z_ld = kH;
+        d.z = w.z[l - 1];
         d.col_sum = w.grads + b_off(l - 1);
         d.img = w.dz_img[cur ^ 1]; d.img_rows = batch;
         d.img_t = w.dz_imgt[cur ^ 1]; d.img_t_rows = kH;
@@ -1445,10 +1506,10 @@ cudaError_t train_step(float* p, uint8_t* img, float* m, float* v, const float* 
     if (e == cudaSuccess) {
         GemmArgs g = gemm_args(w.dz_imgt[cur], kH, w.enc_imgt, kEnc, kchunks/splits);
         g.out = w.ws; g.ld = kEnc; g.split_stride = ws_stride; g.n_store = kEnc;
-        e = launch_gemm<kEnc, kEpiF32>(g, kH, kEnc, splits, s);
+        e = launch_gemm<kEnc>(g, kH, kEnc, splits, s);
     }
     if (e == cudaSuccess) {
-        reduce_dw_kernel<<<148, 256, 0, s>>>(w.ws, splits, ws_stride, kH, kEnc, w.grads + kW0);
+        reduce_dw_kernel<<<(kH*kEnc + 255)/256, 256, 0, s>>>(w.ws, splits, ws_stride, kH, kEnc, w.grads + kW0);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && grads_out)
@@ -1458,7 +1519,7 @@ cudaError_t train_step(float* p, uint8_t* img, float* m, float* v, const float* 
     if (e == cudaSuccess) {
         const double c1 = 1.0/(1.0 - std::pow(0.9, (double)step));
         const double c2 = 1.0/(1.0 - std::pow(0.999, (double)step));
-        adam_kernel<<<148, 256, 0, s>>>(p, w.grads, m, v, kParams, lr, (float)c1, (float)c2);
+        adam_kernel<<<(uint32_t)((kParams + 255)/256), 256, 0, s>>>(p, w.grads, m, v, kParams, lr, (float)c1, (float)c2);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
@@ -1500,9 +1561,9 @@ int mlgpu_sg_gemm_f32(const void* a_img, uint32_t a_rows, const void* b_img, uin
     g.bias = bias; g.bias_n = n; g.out = c; g.ld = n; g.n_store = n;
     const cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
     cudaError_t e;
-    if (n % 256 == 0 && b_rows % 256 == 0) e = launch_gemm<256, kEpiF32>(g, m, n, 1, s);
-    else if (n % 128 == 0 && b_rows % 128 == 0) e = launch_gemm<128, kEpiF32>(g, m, n, 1, s);
-    else if (n == 80 && b_rows == 80) e = launch_gemm<80, kEpiF32>(g, m, n, 1, s);
+    if (n % 256 == 0 && b_rows % 256 == 0) e = launch_gemm<256>(g, m, n, 1, s);
+    else if (n % 128 == 0 && b_rows % 128 == 0) e = launch_gemm<128>(g, m, n, 1, s);
+    else if (n == 80 && b_rows == 80) e = launch_gemm<80>(g, m, n, 1, s);
     else return report_error(MLGPU_ERR_INVALID_ARGUMENT, "n must be 80 or a multiple of 128");
     if (e != cudaSuccess) return report_error(MLGPU_ERR_CUDA, cudaGetErrorString(e));
     return MLGPU_OK;
