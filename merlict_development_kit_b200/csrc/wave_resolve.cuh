@@ -306,7 +306,9 @@ wave_hit_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
             }
             __syncwarp();
         }
-        groups = visit_nodes(sc, sw, stack, lane, groups, &l);
+#pragma unroll 1
+        for (int k = 0; k < kVisits; k++)
+            groups = visit_nodes(sc, sw, stack, lane, groups, &l);
     }
 }
 
