@@ -1,8 +1,7 @@
 // device_sort.cu -- the sorts and scans of the calibration and signal-chain
-// rows: a stable LSD radix sort of (32-bit key, 32-bit value) pairs, a
-// counting sort by a small key, a sort of the long runs of a segmented
-// array by (64-bit key, value) (one block per run), and exclusive sums
-// into 64-bit offsets.
+// rows: a stable LSD radix sort of (32-bit key, 32-bit value) pairs, a sort
+// of the long runs of a segmented array by (64-bit key, value) (one block
+// per run), and exclusive sums into 64-bit offsets.
 //
 // Radix sort, 8-bit digits, one pass per digit (as many as the key bits
 // need), each pass three launches over tiles of kSortTile elements:
@@ -181,6 +180,24 @@ scan_add_kernel(uint64_t* __restrict__ out, uint64_t n, const uint64_t* __restri
     for (uint64_t i = b + threadIdx.x; i < b + kScanTile && i < n; i += blockDim.x) out[i] += add;
 }
 
+// The same with the totals of the blocks before summed here, for as many
+// blocks as a block has threads: the launch that would sum them is most of
+// a short scan (63,380 values: 12.6 us in three launches, 11.1 in two).
+__global__ void __launch_bounds__(kScanThreads)
+scan_spread_kernel(uint64_t* __restrict__ out, uint64_t n, const uint64_t* __restrict__ sums) {
+    __shared__ uint64_t warp_sum[kScanThreads/32];
+    uint64_t add = threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = add;
+    __syncthreads();
+    add = warp_sum[threadIdx.x & 31];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+    const uint64_t b = (uint64_t)blockIdx.x*kScanTile;
+    for (uint64_t i = b + threadIdx.x; i < b + kScanTile && i < n; i += blockDim.x) out[i] += add;
+}
+
 uint64_t scan_levels_words(uint64_t n) {
     uint64_t words = 0;
     while (n > 1) {
@@ -198,6 +215,10 @@ cudaError_t exclusive_sum(const In* in, uint64_t* out, uint64_t n, uint64_t* tem
     scan_tiles_kernel<In><<<(unsigned)blocks, kScanThreads, 0, s>>>(in, n, out, temp);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || blocks == 1) return e;
+    if (blocks <= (uint64_t)kScanThreads) {
+        scan_spread_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(out, n, temp);
+        return cudaGetLastError();
+    }
     // the block totals, summed the same way, then added back
     e = exclusive_sum<uint64_t>(temp, temp, blocks, temp + blocks + 1, s);
     if (e != cudaSuccess) return e;
@@ -273,83 +294,7 @@ segment_sort_kernel(uint64_t* __restrict__ key_in, uint32_t* __restrict__ val_in
     }
 }
 
-// ---- counting sort by a small key --------------------------------------------
-
-// Photons with equal keys within a warp are merged (__match_any_sync): one
-// atomic per key and warp.
-__global__ void __launch_bounds__(256)
-count_keys_kernel(const uint32_t* __restrict__ key, uint64_t n, uint32_t* __restrict__ count) {
-    const int lane = threadIdx.x & 31;
-    for (uint64_t b = (uint64_t)blockIdx.x*blockDim.x + (threadIdx.x & ~31u); b < n;
-         b += (uint64_t)gridDim.x*blockDim.x) {
-        const uint64_t i = b + lane;
-        const bool valid = i < n;
-        const uint32_t k = valid ? __ldg(key + i) : 0u;
-        const unsigned live = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-            const unsigned peers = __match_any_sync(live, k);
-            if (lane == __ffs(peers) - 1) atomicAdd(count + k, (unsigned)__popc(peers));
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256)
-cursor_kernel(const uint64_t* __restrict__ offset, uint32_t keys, uint32_t* __restrict__ cursor) {
-    for (uint32_t k = blockIdx.x*blockDim.x + threadIdx.x; k < keys; k += gridDim.x*blockDim.x)
-        cursor[k] = (uint32_t)offset[k];
-}
-
-__global__ void __launch_bounds__(256)
-place_keys_kernel(const uint32_t* __restrict__ key, uint64_t n, uint32_t* __restrict__ cursor,
-                  uint32_t* __restrict__ index_out) {
-    const int lane = threadIdx.x & 31;
-    for (uint64_t b = (uint64_t)blockIdx.x*blockDim.x + (threadIdx.x & ~31u); b < n;
-         b += (uint64_t)gridDim.x*blockDim.x) {
-        const uint64_t i = b + lane;
-        const bool valid = i < n;
-        const uint32_t k = valid ? __ldg(key + i) : 0u;
-        const unsigned live = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-            const unsigned peers = __match_any_sync(live, k);
-            const int leader = __ffs(peers) - 1;
-            uint32_t first = 0;
-            if (lane == leader) first = atomicAdd(cursor + k, (unsigned)__popc(peers));
-            first = __shfl_sync(peers, first, leader);
-            index_out[first + __popc(peers & ((1u << lane) - 1u))] = (uint32_t)i;
-        }
-    }
-}
-
 }  // namespace
-
-size_t counting_sort_temp_bytes(uint64_t n, uint32_t keys) {
-    // counts and cursors (32-bit, each rounded up to 64 entries), the scan's levels
-    return 2*(((uint64_t)keys + 1 + 63) & ~uint64_t(63))*sizeof(uint32_t) +
-           exclusive_sum_temp_bytes((uint64_t)keys + 1) + 256;
-}
-
-cudaError_t counting_sort(const uint32_t* key, uint64_t n, uint32_t keys, uint32_t* index_out,
-                          uint64_t* offset, void* temp, cudaStream_t s) {
-    if (n >= (1ull << 32)) return cudaErrorInvalidValue;
-    uint32_t* count = static_cast<uint32_t*>(temp);                       // keys + 1
-    uint32_t* cursor = count + (((uint64_t)keys + 1 + 63) & ~uint64_t(63));
-    uint64_t* scan_tmp = reinterpret_cast<uint64_t*>(
-        cursor + (((uint64_t)keys + 1 + 63) & ~uint64_t(63)));
-    cudaError_t e = cudaMemsetAsync(count, 0, ((uint64_t)keys + 1)*sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t want = (n + 255)/256;
-    const unsigned grid = (unsigned)(want < (uint64_t)(8*sms) ? (want ? want : 1) : 8*sms);
-    count_keys_kernel<<<grid, 256, 0, s>>>(key, n, count);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = exclusive_sum<uint32_t>(count, offset, (uint64_t)keys + 1, scan_tmp, s);
-    if (e != cudaSuccess) return e;
-    cursor_kernel<<<(keys + 255)/256, 256, 0, s>>>(offset, keys, cursor);
-    place_keys_kernel<<<grid, 256, 0, s>>>(key, n, cursor, index_out);
-    return cudaGetLastError();
-}
 
 size_t radix_sort_temp_bytes(uint64_t n) {
     const uint64_t tiles = (n + kSortTile - 1)/kSortTile;

@@ -452,13 +452,6 @@ cudaError_t exclusive_sum_u32(const uint32_t* in, uint64_t* out, uint64_t n, voi
 cudaError_t sort_long_runs(uint64_t* key_in, uint32_t* val_in, uint64_t* key_out,
                            uint32_t* val_out, const uint64_t* begin, const uint64_t* end,
                            uint32_t runs, cudaStream_t s);
-// A counting sort by keys in [0, keys): index_out receives the input
-// indices grouped by key (ascending keys; the order within a key is not
-// defined), offset[k] where key k starts (keys + 1 entries, the last the
-// total).  `temp`: counting_sort_temp_bytes(n, keys).  n < 2^32.
-size_t counting_sort_temp_bytes(uint64_t n, uint32_t keys);
-cudaError_t counting_sort(const uint32_t* key, uint64_t n, uint32_t keys, uint32_t* index_out,
-                          uint64_t* offset, void* temp, cudaStream_t s);
 
 // Zeroes counts (and time_hist) and bins n arrivals into them: two kernel
 // launches, no scratch memory (bin.cu).

@@ -4,6 +4,8 @@ Philox draws, and against merlict's own background injection, conversion
 and extraction replaying those draws.  Integer outputs (background photons
 per lixel, pulse offsets, slices, truth ids) and the window start are
 compared exactly."""
+import sys
+
 import numpy as np
 import pytest
 
@@ -89,6 +91,45 @@ def test_gpu_matches_oracle_and_merlict(eng, scene, case):
         assert np.array_equal(off, r["channel_offset"])
         assert np.array_equal(sl, r["channel_slice"])
         assert np.array_equal(trg, r["channel_truth"])
+
+
+@pytest.mark.parametrize("p2,counts", [
+    (0.1, [0, 1, 2, 31, 32, 33, 63, 64, 65, 255, 256, 257, 300]),
+    (0.995, [1, 5, 40]),
+    (0.3, [4095, 4096, 4097]),
+], ids=["run_edges", "long_crosstalk", "pool_edges"])
+def test_equal_times_and_run_lengths(eng, scene, p2, counts):
+    """Runs at the edges of the sorts (one warp up to 256 photons, one block
+    up to 4,096) with equal arrival times, in input order then; crosstalk runs
+    longer than the 255 that a draw's run length counts to; more photons than
+    the 8,192 that a block's shared memory holds.  Whole numbers throughout,
+    so equal ones: the draws, the comparisons and the order are the oracle's
+    in the same arithmetic."""
+    g = geometry()
+    nl = g.num_lixels
+    rng = np.random.default_rng(41)
+    sensor = np.repeat(np.arange(len(counts), dtype=np.int32) % nl, counts)
+    sensor = np.concatenate([sensor, np.full(50, -1, dtype=np.int32)])
+    rng.shuffle(sensor)
+    n = len(sensor)
+    t = 100e-9 + 0.5e-9*rng.integers(0, 40, n).astype(np.float64)
+    w = rng.uniform(300e-9, 600e-9, n)
+    tr = np.arange(n, dtype=np.int32)
+    eff = rng.uniform(0.3, 0.7, nl).astype(np.float32)
+    cfg, light = config(g, p2=p2)
+    off, sl, trg, start, nsb = gpu_chain(eng, scene, cfg, sensor, t, w, tr, eff, 99, 7)
+    limit = sys.getrecursionlimit()
+    sys.setrecursionlimit(20000)       # the oracle calls itself once per crosstalk pulse
+    try:
+        o = SO.signal_chain(sensor, t, w, tr, nl, eff, **chain_kwargs(light, nl, p2=p2))
+    finally:
+        sys.setrecursionlimit(limit)
+    o_off, o_sl, o_tr, *_ = flat(o)
+    assert start == o["nsb_exposure_start_time"]
+    assert np.array_equal(nsb, np.array(o["nsb_count"], dtype=np.int32))
+    assert np.array_equal(off, o_off)
+    assert np.array_equal(sl, o_sl)
+    assert np.array_equal(trg, o_tr)
 
 
 def test_capacity_too_small_is_retried(eng, scene):
