@@ -1201,7 +1201,6 @@ int mlgpu_corsika_photons(mlgpu_scene* scene, const float* bunches, uint64_t n,
     const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
     MLGPU_CUDA(scene->corsika.reserve(corsika_scratch_bytes(n) + 256));
     if (!scene->wave_host) MLGPU_CUDA(cudaMallocHost(&scene->wave_host, sizeof(WaveCounters)));
-    if (!scene->wave_grid) scene->wave_grid = wave_persistent_blocks();
     char* base = static_cast<char*>(scene->corsika.ptr);
     uint64_t* total_dev = reinterpret_cast<uint64_t*>(base);
     void* scratch = base + 256;
@@ -1210,9 +1209,9 @@ int mlgpu_corsika_photons(mlgpu_scene* scene, const float* bunches, uint64_t n,
     r.photon_offset = rng->photon_offset; r.uniforms = rng->uniforms;
     MLGPU_CUDA(cudaMemsetAsync(scene->error_word, 0, sizeof(unsigned int), stream));
     cudaError_t e = launch_corsika_count(bunches, n, r, scratch, total_dev, scene->error_word,
-                                         scene->wave_grid, stream);
+                                         stream);
     if (e != cudaSuccess) return cuda_fail(e, "bunch count kernels");
-    scene->launches += 4;
+    scene->launches += 2;
     // the total and the error word, back on the host (pinned staging)
     uint64_t* host = reinterpret_cast<uint64_t*>(scene->wave_host);
     MLGPU_CUDA(cudaMemcpyAsync(host, total_dev, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream));
@@ -1231,7 +1230,7 @@ int mlgpu_corsika_photons(mlgpu_scene* scene, const float* bunches, uint64_t n,
         return fail(MLGPU_ERR_INVALID_ARGUMENT, "the bunches give %llu photons, the buffers hold %llu",
                     (unsigned long long)total, (unsigned long long)out->capacity);
     e = launch_corsika_expand(bunches, n, bunch_ids, scratch, planes, out->simulation_truth_id,
-                              scene->wave_grid, stream);
+                              stream);
     if (e != cudaSuccess) return cuda_fail(e, "bunch expansion kernel");
     scene->launches += 1;
     return MLGPU_OK;

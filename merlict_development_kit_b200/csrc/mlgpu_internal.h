@@ -364,14 +364,14 @@ cudaError_t launch_trace_fp64(const TraceArgs& a, int block, cudaStream_t s);
 cudaError_t launch_queue_trace(const TraceArgs& a, unsigned long long* queue, int grid,
                                cudaStream_t s);
 int queue_trace_blocks_per_sm();
-// CORSIKA bunches to photons (corsika.cu): counts and offsets into
+// CORSIKA bunches to photons (corsika.cu): counts and their sums into
 // `scratch` (corsika_scratch_bytes), the total to *total_dev; then the
 // expansion into the seven FP64 planes.
 size_t corsika_scratch_bytes(uint64_t n);
 cudaError_t launch_corsika_count(const float* bunches, uint64_t n, const DevRng& rng, void* scratch,
-                                 uint64_t* total_dev, unsigned int* err, int grid, cudaStream_t s);
+                                 uint64_t* total_dev, unsigned int* err, cudaStream_t s);
 cudaError_t launch_corsika_expand(const float* bunches, uint64_t n, const int32_t* ids,
-                                  void* scratch, double* const* planes, int32_t* out_id, int grid,
+                                  void* scratch, double* const* planes, int32_t* out_id,
                                   cudaStream_t s);
 // Per-sensor calibration statistics (lixel_stats.cu): `values` = cx, cy,
 // x, y, time delay; `out` [num_sensors][12].

@@ -112,3 +112,52 @@ def test_event_tape_bunches_through_the_device_factory(tmp_path):
         for k in ("support_x", "support_y", "support_z", "wavelength", "id"):
             assert np.array_equal(got[k].cpu().numpy(), ref[k]), k
     scene.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 255, 256, 257, 1023, 1024, 1025, 5000])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3, -1])
+def test_expansion_at_the_edges_of_its_tiles(n, shift):
+    """The expansion's blocks take 256 bunches and write four photons of a
+    plane at once from 32-byte boundaries: planes that begin `shift` photons
+    past one (-1: each plane elsewhere), bunches and buffers beside which
+    nothing may be written.  The oracle's photons bit for bit."""
+    import ctypes as C
+    import torch
+    from merlict_development_kit_b200 import _native, abi, engine
+    from conftest import load_golden
+    b, u = random_bunches(n, 100 + n)
+    b[n//2:n//2 + 300, 6] = 16.0              # 17 photons where the draw is 0
+    u[n//2:n//2 + 300] = 0.0
+    ref = O.corsika_photons_numpy(b, u)
+    m = len(ref["id"])
+    scene = engine.Scene(load_golden("sphere")[0])
+    flat = torch.zeros(8*n + 1, dtype=torch.float32, device="cuda")
+    flat[1:] = torch.as_tensor(b.reshape(-1), device="cuda")      # rows on 4 bytes only
+    names = PLANES + ("id",)
+    at = {k: 4 + (shift if shift >= 0 else i % 4) for i, k in enumerate(names)}
+    whole = {k: torch.full((m + 12,), -7, device="cuda",
+                           dtype=torch.int32 if k == "id" else torch.float64) for k in names}
+    buf = abi.mlgpu_photon_buffers()
+    for k in PLANES:
+        setattr(buf, k, whole[k].data_ptr() + 8*at[k])
+    buf.simulation_truth_id = whole["id"].data_ptr() + 4*at["id"]
+    buf.capacity = m
+    r, keep = engine.Replay(torch.as_tensor(u[:, None], device="cuda"))._struct(n)
+    num = C.c_uint64()
+    _native.check(_native.lib().mlgpu_corsika_photons(
+        scene.handle, C.c_void_p(flat.data_ptr() + 4), n, None, C.byref(r), C.byref(buf),
+        C.byref(num), C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    del keep
+    assert num.value == m
+    got = {k: v.cpu().numpy() for k, v in whole.items()}
+    for k in names:
+        assert np.all(got[k][:at[k]] == -7) and np.all(got[k][at[k] + m:] == -7), k
+        got[k] = got[k][at[k]:at[k] + m]
+    for k in ("support_x", "support_y", "support_z", "wavelength", "id"):
+        assert np.array_equal(got[k], ref[k]), k
+    d = normalised((got["direction_x"], got["direction_y"], got["direction_z"]))
+    for k, v in zip(("direction_x", "direction_y", "direction_z"), d):
+        assert np.array_equal(v, ref[k]), k
+    scene.close()
