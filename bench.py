@@ -42,26 +42,21 @@ BYTES_PER_PHOTON = {"fp64": 88, "fp64_plain": 88, "fp32": 52}
 # Fresnel steps, time-of-flight segments, table look-ups)
 FLOP_WEIGHTS = {"nodes": 26, "leaves": 48, "caps": 29, "cap_bounds": 85, "planes": 36,
                 "others": 29, "reflections": 91, "fresnels": 110, "segments": 3, "funcs": 4}
-# the kernel class that does each counted operation
-FLOP_STAGE = {"nodes": "walk", "leaves": "intersect", "caps": "intersect",
-              "cap_bounds": "intersect", "planes": "intersect", "others": "intersect",
-              "reflections": "resolve", "fresnels": "resolve", "segments": "resolve",
-              "funcs": "resolve"}
+# the kernel class that does each counted operation (the closest-hit walk
+# intersects the leaves it finds)
+FLOP_STAGE = {"nodes": "walk", "leaves": "walk", "caps": "walk", "cap_bounds": "walk",
+              "planes": "walk", "others": "walk", "reflections": "resolve",
+              "fresnels": "resolve", "segments": "resolve", "funcs": "resolve"}
 FP64_PEAK_TFLOPS_NOMINAL = 37.0   # B200 vector FP64 with FMAs, nominal
 # DRAM bytes per photon of each kernel class on the light-field telescope,
-# from an ncu capture of the timed step of 4e6 photons (dram__bytes_read.sum
+# from an ncu capture of one propagation of 4e6 photons (dram__bytes_read.sum
 # + dram__bytes_write.sum summed over the class's launches, divided by the
-# photons of the step; profiles/wavefront_fp64_light_field_telescope.md):
-# walk = the BVH level kernels; intake = intake + counter kernel;
-# intersect = intersection + tie kernels; resolve = overflow walk +
-# resolve + counter kernel; bin = zeroing + binning kernels.  The tracing
-# order's kernels (run once per call, before the first iteration) are in
-# no class (ORDER_DRAM_BYTES_PER_PHOTON).  The traffic of a step grows with its photons
-# (the same scene and pool), so the bench scales these figures by its own
-# photon count.
-STAGE_DRAM_BYTES_PER_PHOTON = {"walk": 807.0, "intake": 247.5, "intersect": 1079.9,
-                               "resolve": 897.4, "bin": 4.0}
-ORDER_DRAM_BYTES_PER_PHOTON = 188.0
+# photons; profiles/wavefront_fp64_light_field_telescope.md): walk = the
+# closest-hit walks; resolve = the interactions; plain = the first look at
+# every photon and the kernel that ends the last rays; bin = zeroing and
+# binning kernels.  The traffic of a step grows with its photons (the same
+# scene and pool), so the bench scales these figures by its own photon count.
+STAGE_DRAM_BYTES_PER_PHOTON = {"walk": 242.7, "resolve": 650.8, "plain": 64.9, "bin": 4.0}
 FP32_PEAK_TFLOPS_NOMINAL = 75.0   # B200 vector FP32 (non-tensor), nominal
 WORKLOAD = "light-field telescope, 1039 lenses x 61 lixels (config 1)"
 # the signal chain after binning (workload "signal"): quantum efficiency,
@@ -477,9 +472,9 @@ def run_ours(args, world, rank, local):
                                 "MEASURED_PEAKS.json)"),
            "bytes_per_photon": bpp, "scope": "whole propagate call"}
     if STAGE_DRAM_BYTES_PER_PHOTON and not fp32:
-        # the FP64 tracer's measured DRAM traffic (ncu, all kernel classes and
-        # the tracing order) against the algorithmic bytes
-        measured = sum(STAGE_DRAM_BYTES_PER_PHOTON.values()) + ORDER_DRAM_BYTES_PER_PHOTON
+        # the FP64 tracer's measured DRAM traffic (ncu, all kernel classes)
+        # against the algorithmic bytes
+        measured = sum(STAGE_DRAM_BYTES_PER_PHOTON.values())
         hbm["dram_bytes_per_photon_measured"] = measured
         hbm["dram_over_algorithmic"] = measured / bpp
     cpu = None

@@ -289,11 +289,12 @@ int mlgpu_scene_kernel_launches(const mlgpu_scene* scene, uint64_t* launches);
  * reference: it exists so that callers can put a roofline on each stage of
  * the device pipeline.                                                    */
 enum {
-    MLGPU_KERNEL_WALK = 0,       /* BVH levels and leaf-sphere tests          */
-    MLGPU_KERNEL_INTAKE = 1,     /* photon intake, lens walks, pool counters  */
-    MLGPU_KERNEL_INTERSECT = 2,  /* one thread per candidate, closest hit     */
-    MLGPU_KERNEL_RESOLVE = 3,    /* interaction, compaction, results          */
-    MLGPU_KERNEL_PLAIN = 4,      /* one-thread-per-photon tracer              */
+    MLGPU_KERNEL_WALK = 0,       /* closest hits, or BVH levels               */
+    MLGPU_KERNEL_INTAKE = 1,     /* level walk: photon intake, lens walks     */
+    MLGPU_KERNEL_INTERSECT = 2,  /* level walk: one thread per candidate      */
+    MLGPU_KERNEL_RESOLVE = 3,    /* interaction, compaction, results, intake  */
+    MLGPU_KERNEL_PLAIN = 4,      /* one thread per photon: first look, whole  *
+                                  * small batches, last rays, other tracers   */
     MLGPU_KERNEL_BIN = 5,        /* arrival binning                           */
     MLGPU_KERNEL_CLASSES = 6
 };

@@ -1111,11 +1111,13 @@ int mlgpu_scene_autotune(mlgpu_scene* scene, const mlgpu_photons* sample, uint64
     cudaEvent_t ev[2] = {nullptr, nullptr};
     MLGPU_CUDA(cudaEventCreate(&ev[0]));
     MLGPU_CUDA(cudaEventCreate(&ev[1]));
-    // times one setting: best of two runs after an untimed one
+    // times one setting: best of four runs after an untimed one (a sample of
+    // which most photons miss takes about 1 ms, and two runs of that differ by
+    // more than the knobs do)
     auto time_of = [&](const mlgpu_settings& cand, double* ms) -> int {
         const TraceArgs a = make_args(scene, sample, n, &cand, rng, &res);
         double t_best = 1e300;
-        for (int rep = 0; rep < 3; rep++) {
+        for (int rep = 0; rep < 5; rep++) {
             if (cudaEventRecord(ev[0], stream) != cudaSuccess) return cuda_fail(cudaGetLastError(), "event");
             const int r = launch(scene, a, &cand, stream);
             if (r) return r;
@@ -1140,7 +1142,7 @@ int mlgpu_scene_autotune(mlgpu_scene* scene, const mlgpu_photons* sample, uint64
     double cur_ms = 0.0;
     st = time_of(cur, &cur_ms);
     // candidate values of each knob, tried one knob at a time
-    const uint32_t pools[] = {1u << 19, 1u << 20, 1u << 21, 1u << 22};
+    const uint32_t pools[] = {1u << 19, 1u << 20, 1u << 21, 1u << 22, 1u << 23};
     const int periods[] = {2, 4, 8, 16};
     const int grids[] = {4*sms, 8*sms, 16*sms};
     const int stages[] = {0, 3, 5};
@@ -1150,12 +1152,18 @@ int mlgpu_scene_autotune(mlgpu_scene* scene, const mlgpu_photons* sample, uint64
     for (int pass = 0; pass < 2 && st == MLGPU_OK; pass++) {
         const double start_ms = cur_ms;
         for (int knob = 0; knob < 7 && st == MLGPU_OK; knob++) {
-            const int count = knob <= 1 ? 4 : knob <= 3 ? 3 : 2;
+            const int count = knob == 0 ? 5 : knob == 1 ? 4 : knob <= 3 ? 3 : 2;
             for (int c = 0; c < count && st == MLGPU_OK; c++) {
                 mlgpu_settings cand = cur;
                 switch (knob) {
                 case 0:
                     if (pools[c] > 2*n && c > 0) continue;   // larger than the sample
+                    // the closest-hit walk gains with every larger pool (1e7
+                    // telescope photons: 22.4, 19.6, 18.3, 17.7, 17.4 ms), which a
+                    // sample that does not fill them cannot show: small ones,
+                    // chosen for 4e6 mostly missing photons, made 4.4e8 20 % slower
+                    if (pools[c] < (1u << 21) && wave_walk(scene, &cur) == MLGPU_WALK_STACK)
+                        continue;
                     cand.pool_size = pools[c];
                     break;
                 case 1: cand.check_period = periods[c]; break;
@@ -1168,7 +1176,10 @@ int mlgpu_scene_autotune(mlgpu_scene* scene, const mlgpu_photons* sample, uint64
                 if (std::memcmp(&cand, &cur, sizeof(cand)) == 0) continue;
                 double ms = 0.0;
                 st = time_of(cand, &ms);
-                if (st == MLGPU_OK && ms < cur_ms) { cur = cand; cur_ms = ms; }
+                // a knob moves from its default for 2 % or more: two runs of one
+                // setting differ by up to 1 %, and a pool size fixed for a sample
+                // of 2e6 photons by less than that made 1e7 take 17.3 ms, not 16.8
+                if (st == MLGPU_OK && ms < 0.98*cur_ms) { cur = cand; cur_ms = ms; }
             }
         }
         if (cur_ms > 0.98*start_ms) break;   // the pass gained little

@@ -2,8 +2,15 @@
 // (merlict/PhotonAndFrame.cpp:13-124) split into per-step kernels over a
 // fixed pool of ray slots, bit-identical to the plain tracer.
 //
-// One iteration over the pool, every stage a flat loop over uniform work
-// items so that a warp's lanes do the same thing:
+// By default an iteration over the pool is two kernels: the closest hit of
+// every ray (closest_hit.cuh), then its interaction, which also takes new
+// photons into the slots that come free (wave_resolve.cuh).  Photons that
+// miss the scenery end in a first look, before the pool; small batches and
+// the last rays of large ones are traced to their ends by one launch.
+//
+// The level kernels are the other walk, for scenes without a surface BVH, for
+// the caller's own queue capacity and for merlict's walks in single precision
+// alone; every stage a flat loop over uniform work items:
 //   intake     one thread per slot: new photons enter free slots; a ray
 //              inside a lens gets merlict's walk of that lens's subtree
 //              (RayAndFrame.cpp:137-149), every other ray queues the root
@@ -13,8 +20,6 @@
 //              the leaves of hit leaf ranges that pass a conservative FP32
 //              version of merlict's bounding-sphere test become candidates
 //              (merlict's exact test follows in the intersection step);
-//   (or walk   one thread per ray: levels and sphere tests in one
-//              depth-first walk with a stack, the same candidates;)
 //   intersect, ties, overflow, resolve: wave_resolve.cuh.
 // The arithmetic is the shared FP64 code, compiled with --fmad=false.
 #include <cstdint>
