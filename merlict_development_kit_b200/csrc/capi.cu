@@ -1404,9 +1404,11 @@ int mlgpu_signal_chain(mlgpu_scene* scene, const mlgpu_signal_chain_config* cfg,
 int mlgpu_scene_sync_errors(mlgpu_scene* scene, void* cuda_stream) {
     if (!scene) return fail(MLGPU_ERR_INVALID_ARGUMENT, "scene is NULL");
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-    MLGPU_CUDA(cudaStreamSynchronize(s));
     unsigned int code = 0;
-    MLGPU_CUDA(cudaMemcpy(&code, scene->error_word, sizeof(code), cudaMemcpyDeviceToHost));
+    // queued behind the stream's work: the host waits once, not for the work
+    // and then for a copy
+    MLGPU_CUDA(cudaMemcpyAsync(&code, scene->error_word, sizeof(code), cudaMemcpyDeviceToHost, s));
+    MLGPU_CUDA(cudaStreamSynchronize(s));
     if (code) {
         MLGPU_CUDA(cudaMemset(scene->error_word, 0, sizeof(unsigned int)));
         return fail((int)code, "%s", device_error_text(code));
