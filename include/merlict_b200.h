@@ -277,7 +277,13 @@ int mlgpu_last_error(char* buffer, size_t buffer_size);
  * Replaces the per-call frame-tree walk of CausalIntersection
  * (merlict/RayAndFrame.cpp:126-173) by a device copy of the tree.
  * Validates the flat scene (index ranges, sorted tables) and uploads it to
- * the current CUDA device.                                              */
+ * the current CUDA device.
+ * A scene owns scratch memory that its calls share: ray pools, photon lists,
+ * sort buffers, counters, the error word.  One host thread at a time uses a
+ * scene.  Its calls may name different streams: one that writes the scratch
+ * starts on the device after what earlier calls left in flight on other
+ * streams, without a wait on the host.  Calls captured into a graph are not
+ * ordered so; a graph that holds calls on a scene is the caller's to order. */
 int mlgpu_scene_create(const mlgpu_flat_scene* flat, mlgpu_scene** scene);
 int mlgpu_scene_destroy(mlgpu_scene* scene);
 
@@ -336,7 +342,9 @@ int mlgpu_probe_fp64_rate(int fma, double* flops_per_second, void* cuda_stream);
  * Replaces propagate_photons_in_frame_with_config (merlict/Photons.cpp:9-22)
  * and its thread-pool twin (merlict_multi_thread.cpp:28-55).
  * Device pointers, asynchronous on `cuda_stream` (a cudaStream_t, NULL =
- * default stream).  Errors found on the device (a wavelength outside a
+ * default stream): the call may return before its last kernels have run, so
+ * inputs, results and a replay table stay as they are until the stream has
+ * passed them.  Errors found on the device (a wavelength outside a
  * property table, an exhausted replay stream) are reported by
  * mlgpu_scene_sync_errors().                                             */
 int mlgpu_propagate(

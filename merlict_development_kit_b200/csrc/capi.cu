@@ -9,6 +9,7 @@
 #include <mutex>
 #include <vector>
 
+#include "in_flight.h"
 #include "mlgpu_internal.h"
 
 using namespace mlgpu;
@@ -143,6 +144,7 @@ struct mlgpu_scene {
     void* arena = nullptr;           // the scene's read-only arrays, one allocation
     size_t arena_bytes = 0;
     unsigned int* error_word = nullptr;
+    InFlight in_flight;              // calls whose last kernels may still use what follows
     // staging for mlgpu_propagate_host and scratch for binning
     DeviceBuffer staging_in, staging_out, staging_hist, staging_rng, tune_out;
     DeviceBuffer staging_bins;           // counts and time histograms of a host call
@@ -698,7 +700,8 @@ struct FeedPlan {
 // against 18.30 ms), smaller and sparser batches lose by it (80,000 photons
 // 467 against 563 us, 25e6 photons of air showers 3.8 against 5.6 ms, 8e6 of
 // the large reflector in FP32 5.3 against 6.2 ms).
-int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, cudaStream_t stream, bool* done) {
+int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, bool whole, cudaStream_t stream,
+               bool* done) {
     WaveBuffers w;
     RayPool none;
     std::memset(&w, 0, sizeof(w));
@@ -706,7 +709,6 @@ int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, cudaStream_t str
     w.walk = MLGPU_WALK_STACK;
     w.fn_smem_bytes = table_smem_bytes(scene);
     const uint64_t n = a->num_photons;
-    const bool whole = n <= std::min(kFinishRays, want);
     if (!whole && n >= (1ull << 31)) return MLGPU_OK;
     Profiler::Chain ch;
     const bool timed = scene->prof.on && scene->prof.take(2, ch.ev);
@@ -764,15 +766,19 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     const bool finish = walk == MLGPU_WALK_STACK && form == MLGPU_TRACER_FP64;
     const uint32_t want = st->pool_size ? st->pool_size
         : walk == MLGPU_WALK_STACK && !feed ? kWalkPool : kWavePool;
+    const bool look = finish && !feed && st->photon_order != MLGPU_ORDER_COHERENT;
+    const bool whole = look && a.num_photons <= std::min(kFinishRays, want);
+    // but for a batch of one launch, the call writes the scene's scratch
+    if (!whole) MLGPU_CUDA(scene->in_flight.wait(stream));
     if (feed) {
         a.sorted = feed->records;
         a.order = nullptr;
         a.fed = 1;
         a.feed_chunks = feed->pieces;
         for (int c = 0; c <= feed->pieces; c++) a.feed_start[c] = feed->start[c];
-    } else if (finish && st->photon_order != MLGPU_ORDER_COHERENT) {
+    } else if (look) {
         bool done = false;
-        const int r = first_look(scene, &a, want, stream, &done);
+        const int r = first_look(scene, &a, want, whole, stream, &done);
         if (r || done) return r;
     } else if (walk != MLGPU_WALK_STACK || st->photon_order == MLGPU_ORDER_COHERENT) {
         const int ro = tracing_order(scene, &a, st, stream, true);
@@ -910,8 +916,8 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     return MLGPU_OK;
 }
 
-int launch(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
-           cudaStream_t stream) {
+int launch_tracer(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
+                  cudaStream_t stream) {
     cudaError_t e;
     switch (st->tracer) {
     case MLGPU_TRACER_FP64:
@@ -919,6 +925,7 @@ int launch(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
     case MLGPU_TRACER_FP32_PURE: return run_wavefront(scene, a, st, stream);
     case MLGPU_TRACER_FP64_QUEUE: {
         TraceArgs q = a;
+        MLGPU_CUDA(scene->in_flight.wait(stream));
         const int ro = tracing_order(scene, &q, st, stream, false);
         if (ro) return ro;
         MLGPU_CUDA(scene->queue.reserve(256));
@@ -956,6 +963,15 @@ int launch(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
     }
     if (e != cudaSuccess) return cuda_fail(e, "trace kernel launch");
     return MLGPU_OK;
+}
+
+// One propagation, its last kernels left in flight.
+int launch(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
+           cudaStream_t stream) {
+    const int rc = launch_tracer(scene, a, st, stream);
+    const cudaError_t e = scene->in_flight.mark(stream);
+    if (rc == MLGPU_OK && e != cudaSuccess) return cuda_fail(e, "event behind a propagation");
+    return rc;
 }
 
 const char* device_error_text(unsigned int code) {
@@ -1068,6 +1084,7 @@ int mlgpu_scene_destroy(mlgpu_scene* scene) {
     scene->corsika.release();
     scene->stats.release();
     scene->wave.release();
+    scene->in_flight.release();
     if (scene->wave_host) cudaFreeHost(scene->wave_host);
     if (scene->wave_graph) cudaGraphExecDestroy(scene->wave_graph);
     if (scene->capture_stream) cudaStreamDestroy(scene->capture_stream);

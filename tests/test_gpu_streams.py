@@ -1,0 +1,88 @@
+"""One scene used from several streams: a call returns while its last kernels
+still use the scene's scratch (csrc/in_flight.h), and the next call, on
+whatever stream, comes after them.  Every result is compared bit for bit
+with the same calls one by one."""
+import numpy as np
+import pytest
+
+from conftest import load_golden
+from merlict_development_kit_b200 import abi, photons as P
+
+pytestmark = pytest.mark.gpu
+
+OUT = ("sensor", "x", "y", "time", "final_leaf", "info")
+
+
+@pytest.fixture(scope="module")
+def telescope():
+    from merlict_development_kit_b200 import engine
+    flat, _, _, meta = load_golden("light_field_small")
+    scene = engine.Scene(flat)
+    yield scene, meta["max_interactions"]
+    scene.close()
+
+
+def equal(a, b):
+    import torch
+    return all(torch.equal(a[k].view(torch.uint8), b[k].view(torch.uint8)) for k in OUT)
+
+
+@pytest.mark.parametrize("tracer,n", [("fp64", 300_001), ("fp64_queue", 100_003), ("fp32", 300_001),
+                                      ("fp64", 20_011)])
+def test_two_batches_on_two_streams(telescope, tracer, n):
+    """More photons than one launch takes, so the pools are used: the second
+    call clears and refills them while the first one's last rays are traced."""
+    import torch
+    from merlict_development_kit_b200 import engine
+    scene, depth = telescope
+    config = engine.PropagationConfig(depth)
+    batches = [engine.photons_to_device(P.downward_disc_source(n + k, 5 + k, 5.55, 21.4, 0.5))
+               for k in range(4)]
+    kw = dict(outputs=OUT, tracer=tracer)
+    one_by_one = [scene.propagate(b, config, engine.Philox(k), **kw) for k, b in enumerate(batches)]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = [scene.propagate(b, config, engine.Philox(k), stream=streams[k % 3], sync=False, **kw)
+               for k, b in enumerate(batches)]
+        torch.cuda.synchronize()
+        assert [equal(a, b) for a, b in zip(one_by_one, got)] == [True]*4
+
+
+def test_a_host_call_behind_a_stream(telescope):
+    """The host-buffer call runs on streams of its own."""
+    import ctypes as C
+    import torch
+    from merlict_development_kit_b200 import engine
+    from merlict_development_kit_b200._native import check, lib
+    scene, depth = telescope
+    n = 2_200_000
+    config = engine.PropagationConfig(depth)
+    first = engine.photons_to_device(P.downward_disc_source(300_001, 1, 5.55, 21.4, 0.5))
+    batch = P.downward_disc_source(n, 2, 5.55, 21.4, 0.5)
+    kw = dict(outputs=OUT)
+    want_first = scene.propagate(first, config, engine.Philox(1), **kw)
+    dev = engine.photons_to_device(batch)
+    want = scene.propagate(dev, config, engine.Philox(2), outputs=("sensor", "time"))
+    host = {k: torch.from_numpy(np.ascontiguousarray(batch[k], np.float64)).pin_memory()
+            for k in P.PLANES}
+    sensor = torch.empty(n, dtype=torch.int32).pin_memory()
+    time = torch.empty(n, dtype=torch.float64).pin_memory()
+    ph = abi.mlgpu_photons()
+    ph.dtype = abi.F64
+    for k in P.PLANES:
+        setattr(ph, k, host[k].data_ptr())
+    res = abi.mlgpu_results()
+    res.dtype = abi.F64
+    res.sensor, res.time = sensor.data_ptr(), time.data_ptr()
+    st = engine._settings(config, 0, "fp64", "bvh", None)
+    r, _ = engine.Philox(2)._struct(n)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got_first = scene.propagate(first, config, engine.Philox(1), stream=stream, sync=False, **kw)
+    check(lib().mlgpu_propagate_host(scene.handle, C.byref(ph), n, C.byref(st), C.byref(r),
+                                     C.byref(res)))
+    torch.cuda.synchronize()
+    assert equal(want_first, got_first)
+    assert torch.equal(sensor, want["sensor"].cpu())
+    assert torch.equal(time.view(torch.int64), want["time"].cpu().view(torch.int64))
