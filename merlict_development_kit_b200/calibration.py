@@ -62,10 +62,14 @@ def lixel_statistics(scene: engine.Scene, sensor: torch.Tensor, cx, cy, x, y, ti
     arrays = [sensor.to(torch.int32).contiguous()] + [
         a.to(torch.float32).contiguous() for a in (cx, cy, x, y, time_delay)]
     out = torch.empty((scene.num_sensors, 12), dtype=torch.float32, device=sensor.device)
-    check(lib().mlgpu_lixel_statistics(scene.handle, *[C.c_void_p(a.data_ptr()) for a in arrays],
-                                       n, float(photons_emitted_per_lixel),
-                                       C.c_void_p(out.data_ptr()),
-                                       C.c_void_p(engine._stream_handle(stream))))
+    engine._behind_current(stream)
+    rc = lib().mlgpu_lixel_statistics(scene.handle, *[C.c_void_p(a.data_ptr()) for a in arrays],
+                                      n, float(photons_emitted_per_lixel),
+                                      C.c_void_p(out.data_ptr()),
+                                      C.c_void_p(engine._stream_handle(stream)))
+    engine._in_use(stream, *arrays, out)
+    check(rc)
+    engine._behind_call(stream)
     o = out.cpu().numpy()
     return {f: o[:, k] for k, f in enumerate(FIELDS)}
 

@@ -75,6 +75,41 @@ def _stream_handle(stream) -> int:
     return int(s.cuda_stream)
 
 
+def _elsewhere(stream):
+    """`stream` as a torch stream if a call on it leaves the current one."""
+    if stream is None or int(stream.cuda_stream) == int(torch.cuda.current_stream().cuda_stream):
+        return None
+    return (stream if isinstance(stream, torch.cuda.Stream)
+            else torch.cuda.ExternalStream(int(stream.cuda_stream)))
+
+
+def _behind_current(stream) -> None:
+    """For a call on `stream` that uses tensors made here (results, converted
+    inputs, a copied table): it starts after the current stream's work so
+    far, where they are filled and where their memory was last in use."""
+    s = _elsewhere(stream)
+    if s is not None:
+        s.wait_stream(torch.cuda.current_stream())
+
+
+def _in_use(stream, *tensors) -> None:
+    """Keeps the memory of `tensors` from being given out again until
+    `stream` has passed the work queued on it: a call returns before its
+    kernels have run."""
+    s = _elsewhere(stream)
+    if s is not None:
+        for t in tensors:
+            if t is not None:
+                t.record_stream(s)
+
+
+def _behind_call(stream) -> None:
+    """The current stream's next work comes after the call on `stream`."""
+    s = _elsewhere(stream)
+    if s is not None:
+        torch.cuda.current_stream().wait_stream(s)
+
+
 def photons_to_device(batch: dict, dtype=torch.float64) -> dict:
     """Copies a photon batch (numpy or torch) to the current CUDA device."""
     out = {}
@@ -174,24 +209,32 @@ class Scene:
             "final_direction": ((n, 3), torch.float64),
         }
         wanted = set(outputs) | {"sensor"}
+        made = history
+        used = [photons[k] for k in PLANES]
         for k, (shape, dt) in spec.items():
             if k in wanted:
                 if k not in out or out[k].shape[0] < n:
                     out[k] = torch.empty(shape, dtype=dt, device=dev)
+                    made = True
                 setattr(res, k, out[k].data_ptr())
+                used.append(out[k])
         if history:
             m = config.max_num_interactions_per_photon + 1
             out["history"] = torch.empty((n, m, abi.HISTORY_DTYPE.itemsize), dtype=torch.uint8, device=dev)
             res.history = out["history"].data_ptr()
+            used.append(out["history"])
         st = _settings(config, start_node, tracer, traversal, tuning)
         r, keep = rng._struct(n)
+        if made or (keep is not None and keep is not rng.uniforms):
+            _behind_current(stream)
         sh = _stream_handle(stream)
-        check(lib().mlgpu_propagate(self._h, C.byref(ph), n, C.byref(st), C.byref(r),
-                                    C.byref(res), C.c_void_p(sh)))
+        rc = lib().mlgpu_propagate(self._h, C.byref(ph), n, C.byref(st), C.byref(r),
+                                   C.byref(res), C.c_void_p(sh))
+        _in_use(stream, keep, *used)
+        check(rc)
         rng.advance(n)
         if sync:
             check(lib().mlgpu_scene_sync_errors(self._h, C.c_void_p(sh)))
-        del keep
         return out
 
     def autotune(self, photons: dict, config: PropagationConfig | None = None,
@@ -207,6 +250,8 @@ class Scene:
         best = abi.mlgpu_settings()
         ms = C.c_double(0.0)
         r, keep = rng._struct(n)
+        if keep is not None:
+            _behind_current(stream)
         check(lib().mlgpu_scene_autotune(self._h, C.byref(ph), n, C.byref(base), C.byref(r),
                                          C.byref(best), C.byref(ms),
                                          C.c_void_p(_stream_handle(stream))))
@@ -237,12 +282,14 @@ class Scene:
         buf.capacity = cap
         total = C.c_uint64(0)
         ids = bunch_ids.contiguous() if bunch_ids is not None else None
-        check(lib().mlgpu_corsika_photons(self._h, C.c_void_p(b.data_ptr()), n,
-                                          C.c_void_p(ids.data_ptr() if ids is not None else None),
-                                          C.byref(r), C.byref(buf), C.byref(total),
-                                          C.c_void_p(_stream_handle(stream))))
+        _behind_current(stream)
+        rc = lib().mlgpu_corsika_photons(self._h, C.c_void_p(b.data_ptr()), n,
+                                         C.c_void_p(ids.data_ptr() if ids is not None else None),
+                                         C.byref(r), C.byref(buf), C.byref(total),
+                                         C.c_void_p(_stream_handle(stream)))
+        _in_use(stream, b, ids, keep, *out.values())
+        check(rc)
         rng.advance(n)
-        del keep
         t = int(total.value)
         return {k: v[:t] for k, v in out.items()}
 
@@ -291,10 +338,13 @@ class Scene:
             hist = torch.empty((self.num_sensors, num_time_bins), dtype=torch.int32,
                                device=sensor.device)
             tp = time.data_ptr()
-        check(lib().mlgpu_bin_arrivals(
+        _behind_current(stream)
+        rc = lib().mlgpu_bin_arrivals(
             self._h, C.c_void_p(sensor.data_ptr()), C.c_void_p(tp), n,
             C.c_void_p(counts.data_ptr()), C.c_void_p(hist.data_ptr() if hist is not None else None),
-            int(num_time_bins), float(t_min), float(t_max), C.c_void_p(_stream_handle(stream))))
+            int(num_time_bins), float(t_min), float(t_max), C.c_void_p(_stream_handle(stream)))
+        _in_use(stream, sensor, time if tp is not None else None, counts, hist)
+        check(rc)
         return counts, hist
 
 

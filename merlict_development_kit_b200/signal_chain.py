@@ -290,7 +290,7 @@ def run(scene, cfg: SignalChainConfig, sensor, arrival_time, wavelength, truth_i
     import torch
 
     from . import _native
-    from .engine import _stream_handle
+    from .engine import _behind_current, _in_use, _stream_handle
     dev = sensor.device
     n = int(sensor.numel())
     num_sensors = int(lixel_efficiency.numel())
@@ -312,9 +312,11 @@ def run(scene, cfg: SignalChainConfig, sensor, arrival_time, wavelength, truth_i
         out.simulation_truth_id = tr.data_ptr()
         out.nsb_count = nsb.data_ptr()
         out.capacity = cap
+        _behind_current(stream)
         rc = _native.lib().mlgpu_signal_chain(
             scene.handle, C.byref(c), *[C.c_void_p(a.data_ptr()) for a in args[:4]], n,
             C.c_void_p(args[4].data_ptr()), num_sensors, C.byref(r), C.byref(out), sh)
+        _in_use(stream, *args, off, sl, tr, nsb)
         if rc == abi.ERR_INVALID_ARGUMENT and out.num_pulses > cap:
             cap = int(out.num_pulses)
             continue

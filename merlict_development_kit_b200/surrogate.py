@@ -62,9 +62,12 @@ def from_image(img: torch.Tensor, rows: int, k: int) -> torch.Tensor:
 def gemm(a_img, a_rows, b_img, b_rows, m, n, k_chunks, bias=None, stream=None) -> torch.Tensor:
     """C = A B^T on the tensor cores (mlgpu_sg_gemm_f32)."""
     c = torch.empty((m, n), dtype=torch.float32, device=a_img.device)
-    check(lib().mlgpu_sg_gemm_f32(a_img.data_ptr(), a_rows, b_img.data_ptr(), b_rows, m, n,
-                                  k_chunks, bias.data_ptr() if bias is not None else None,
-                                  c.data_ptr(), engine._stream_handle(stream)))
+    engine._behind_current(stream)
+    rc = lib().mlgpu_sg_gemm_f32(a_img.data_ptr(), a_rows, b_img.data_ptr(), b_rows, m, n,
+                                 k_chunks, bias.data_ptr() if bias is not None else None,
+                                 c.data_ptr(), engine._stream_handle(stream))
+    engine._in_use(stream, a_img, b_img, bias, c)
+    check(rc)
     return c
 
 

@@ -86,3 +86,33 @@ def test_a_host_call_behind_a_stream(telescope):
     assert equal(want_first, got_first)
     assert torch.equal(sensor, want["sensor"].cpu())
     assert torch.equal(time.view(torch.int64), want["time"].cpu().view(torch.int64))
+
+
+def test_a_calls_tensors_outlive_it(telescope):
+    """What a call on another stream reads or writes stays its own until that
+    stream has passed it, although the caller lets go of it at once."""
+    import torch
+    from merlict_development_kit_b200 import engine
+    scene, depth = telescope
+    n = 20_011
+    config = engine.PropagationConfig(depth)
+    table = np.random.default_rng(3).random((n, 64))
+    batch = P.downward_disc_source(n, 9, 5.55, 21.4, 0.5)
+    want = scene.propagate(engine.photons_to_device(batch), config, engine.Replay(table), outputs=OUT)
+    stream = torch.cuda.Stream()
+    for _ in range(3):
+        photons = engine.photons_to_device(batch)
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)      # some 10 ms in front of the call
+        got = scene.propagate(photons, config, engine.Replay(table), outputs=OUT, stream=stream,
+                              sync=False)
+        dropped = scene.propagate(photons, config, engine.Philox(1), outputs=OUT, stream=stream,
+                                  sync=False)
+        sizes = [t.shape for t in photons.values()] + [t.shape for t in dropped.values()]
+        del photons, dropped
+        filled = [torch.full(s, 7.0, dtype=torch.float64, device="cuda") for s in sizes]
+        filled += [torch.full(table.shape, 7.0, dtype=torch.float64, device="cuda") for _ in range(2)]
+        torch.cuda.synchronize()
+        assert equal(want, got)
+        assert all(bool((t == 7.0).all()) for t in filled)
+        del filled
