@@ -1422,8 +1422,9 @@ int mlgpu_scene_sync_errors(mlgpu_scene* scene, void* cuda_stream) {
     if (!scene) return fail(MLGPU_ERR_INVALID_ARGUMENT, "scene is NULL");
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
     unsigned int code = 0;
-    // queued behind the stream's work: the host waits once, not for the work
-    // and then for a copy
+    // behind the stream's work and what calls on other streams left in
+    // flight: the host waits once, not for the work and then for a copy
+    MLGPU_CUDA(scene->in_flight.wait(s));
     MLGPU_CUDA(cudaMemcpyAsync(&code, scene->error_word, sizeof(code), cudaMemcpyDeviceToHost, s));
     MLGPU_CUDA(cudaStreamSynchronize(s));
     if (code) {

@@ -116,3 +116,28 @@ def test_a_calls_tensors_outlive_it(telescope):
         assert equal(want, got)
         assert all(bool((t == 7.0).all()) for t in filled)
         del filled
+
+
+@pytest.mark.parametrize("n", [300, 300_001])
+def test_errors_of_a_call_on_another_stream(n):
+    """sync_errors reports what earlier propagations raised, whichever stream
+    they were on, also when they are still waiting for their turn there."""
+    import torch
+    from merlict_development_kit_b200 import engine
+    flat, _, _, meta = load_golden("mirror_absorber")
+    scene = engine.Scene(flat)
+    config = engine.PropagationConfig(5)
+    good = engine.photons_to_device(P.isotropic_shell_source(n, 1, 4.0, 2.5))
+    bad = {k: v.clone() for k, v in good.items()}
+    bad["wavelength"][:] = 1500e-9
+    stream = torch.cuda.Stream()
+    for _ in range(2):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)
+        scene.propagate(bad, config, engine.Philox(1), stream=stream, sync=False)
+        with pytest.raises(IndexError):
+            scene.sync_errors()
+        scene.sync_errors(stream=stream)        # reported once
+        scene.propagate(good, config, engine.Philox(1))
+    scene.close()
