@@ -356,7 +356,7 @@ int mlgpu_propagate(
     mlgpu_results* results,
     void* cuda_stream);
 
-/* Waits for `cuda_stream` and for the propagations of this scene before, on
+/* Waits for `cuda_stream` and for the calls on this scene before, on
  * whatever stream, and returns the first device-side error raised since the
  * previous call (then clears it).                                         */
 int mlgpu_scene_sync_errors(mlgpu_scene* scene, void* cuda_stream);

@@ -175,6 +175,23 @@ struct mlgpu_scene {
 
 namespace {
 
+// An entry point's turn at the scene's scratch: it starts after what earlier
+// calls left in flight, and however it ends, what it has queued by then is
+// in flight, unless it has waited for that itself.
+class ScratchTurn {
+ public:
+    ScratchTurn(mlgpu_scene* scene, cudaStream_t stream) : scene_(scene), stream_(stream) {}
+    ~ScratchTurn() { if (scene_) scene_->in_flight.mark(stream_); }
+    ScratchTurn(const ScratchTurn&) = delete;
+    ScratchTurn& operator=(const ScratchTurn&) = delete;
+    cudaError_t wait() { return scene_->in_flight.wait(stream_); }
+    void nothing_left() { scene_ = nullptr; }
+
+ private:
+    mlgpu_scene* scene_;
+    cudaStream_t stream_;
+};
+
 // The scene's arrays are staged on the host while the scene is built and
 // then copied into one device allocation (the scene arena), so that a single
 // L2 access-policy window covers all of them.
@@ -1227,6 +1244,8 @@ int mlgpu_corsika_photons(mlgpu_scene* scene, const float* bunches, uint64_t n,
     for (double* p : planes)
         if (!p) return fail(MLGPU_ERR_INVALID_ARGUMENT, "photon buffer is NULL");
     const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    ScratchTurn turn(scene, stream);
+    MLGPU_CUDA(turn.wait());
     MLGPU_CUDA(scene->corsika.reserve(corsika_scratch_bytes(n) + 256));
     if (!scene->wave_host) MLGPU_CUDA(cudaMallocHost(&scene->wave_host, sizeof(WaveCounters)));
     char* base = static_cast<char*>(scene->corsika.ptr);
@@ -1276,6 +1295,8 @@ int mlgpu_lixel_statistics(mlgpu_scene* scene, const int32_t* sensor, const floa
     if (!(emitted > 0.0))
         return fail(MLGPU_ERR_INVALID_ARGUMENT, "photons_emitted_per_lixel must be > 0");
     const size_t bytes = lixel_stats_scratch_bytes(n);
+    ScratchTurn turn(scene, static_cast<cudaStream_t>(cuda_stream));
+    MLGPU_CUDA(turn.wait());
     MLGPU_CUDA(scene->stats.reserve(bytes));
     if (!scene->wave_grid) scene->wave_grid = wave_persistent_blocks();
     const float* values[5] = {cx, cy, x, y, time_delay};
@@ -1317,6 +1338,8 @@ int mlgpu_signal_chain(mlgpu_scene* scene, const mlgpu_signal_chain_config* cfg,
     if (cfg->num_lixel == 0 || !(cfg->time_slice_duration != 0.0))
         return fail(MLGPU_ERR_INVALID_ARGUMENT, "num_lixel and time_slice_duration must not be 0");
     const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+    ScratchTurn turn(scene, stream);
+    MLGPU_CUDA(turn.wait());
     // the two Func1 tables, on the device
     const size_t nq = cfg->num_quantum_efficiency, nc = cfg->num_nsb_wavelength_cdf;
     MLGPU_CUDA(scene->signal_tables.reserve(3*(nq + nc)*sizeof(double)));
@@ -1413,6 +1436,7 @@ int mlgpu_signal_chain(mlgpu_scene* scene, const mlgpu_signal_chain_config* cfg,
         st = read_back(kept_dev);
         if (st) return st;
         kept = host[0];
+        turn.nothing_left();
     }
     out->num_pulses = kept;
     return MLGPU_OK;

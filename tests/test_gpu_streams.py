@@ -141,3 +141,60 @@ def test_errors_of_a_call_on_another_stream(n):
         scene.sync_errors(stream=stream)        # reported once
         scene.propagate(good, config, engine.Philox(1))
     scene.close()
+
+
+def test_bunches_on_two_streams(telescope):
+    """The expansion reads counts of the scene's scratch, which the next call
+    writes."""
+    import torch
+    from merlict_development_kit_b200 import engine
+    from test_corsika import random_bunches
+    scene, _ = telescope
+    events = [torch.as_tensor(random_bunches(n, k)[0], device="cuda")
+              for k, n in enumerate((400_003, 300_001, 400_009))]
+    want = [scene.corsika_photons(b, engine.Philox(k)) for k, b in enumerate(events)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        got = [scene.corsika_photons(b, engine.Philox(k), stream=streams[k % 2])
+               for k, b in enumerate(events)]
+        torch.cuda.synchronize()
+        for a, b in zip(want, got):
+            assert all(torch.equal(a[k], b[k]) for k in (*P.PLANES, "id"))
+
+
+def test_statistics_on_two_streams(telescope):
+    import ctypes as C
+    import torch
+    from merlict_development_kit_b200._native import check, lib
+    scene, _ = telescope
+    ns = scene.num_sensors
+    sets = []
+    for k, n in enumerate((2_000_003, 1_000_001)):
+        g = torch.Generator(device="cuda").manual_seed(k)
+        sensor = torch.randint(-1, ns, (n,), dtype=torch.int32, device="cuda", generator=g)
+        values = [torch.randn(n, dtype=torch.float32, device="cuda", generator=g) for _ in range(5)]
+        sets.append((n, sensor, values))
+
+    def call(k, stream):
+        n, sensor, values = sets[k]
+        out = torch.empty((ns, 12), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        return out, lambda: check(lib().mlgpu_lixel_statistics(
+            scene.handle, C.c_void_p(sensor.data_ptr()),
+            *[C.c_void_p(v.data_ptr()) for v in values], n, n/ns, C.c_void_p(out.data_ptr()),
+            C.c_void_p(stream.cuda_stream)))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    want = []
+    for k in range(2):
+        out, run = call(k, streams[0])
+        run()
+        torch.cuda.synchronize()
+        want.append(out)
+    for _ in range(3):
+        calls = [call(k, streams[k]) for k in range(2)]
+        for _, run in calls:
+            run()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a.view(torch.int32), c[0].view(torch.int32))
+                   for a, c in zip(want, calls))
