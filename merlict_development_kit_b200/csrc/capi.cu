@@ -1100,6 +1100,9 @@ int mlgpu_scene_destroy(mlgpu_scene* scene) {
     scene->queue.release();
     scene->corsika.release();
     scene->stats.release();
+    scene->signal.release();
+    scene->signal_pulses.release();
+    scene->signal_tables.release();
     scene->wave.release();
     scene->in_flight.release();
     if (scene->wave_host) cudaFreeHost(scene->wave_host);

@@ -189,3 +189,23 @@ def test_full_light_field_sensor_event(eng, scene):
         a, b = int(off[lix]), int(off[lix + 1])
         assert [s for s, _ in x] == list(sl[a:b])
         assert [i for _, i in x] == list(trg[a:b])
+
+
+def test_a_closed_scene_gives_its_memory_back(eng):
+    """The chain's scratch goes with the scene."""
+    import torch
+    from conftest import load_golden
+    flat_scene, *_ = load_golden("sphere")
+    g = geometry()
+    cfg, _ = config(g)
+    ev = event(3, 500_000, g.num_lixels, 3e-9, None)
+
+    def cycle():
+        s = eng.Scene(flat_scene)
+        gpu_chain(eng, s, cfg, *ev, 99, 7)
+        s.close()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+    first = cycle()
+    # each cycle's scratch is some 30 MB
+    assert [cycle() for _ in range(4)][-1] >= first - (4 << 20)
