@@ -488,6 +488,8 @@ void build_surface_bvh(const mlgpu_flat_scene* f, SurfBvhHost* out) {
     for (int32_t i = 0; i < n; i++) b.order[i] = i;
     b.nodes.reserve(2*(size_t)n);
     b.build(0, n, 0);
+    for (int k = 0; k < 3; k++)
+        if (b.nodes[0].box.hi[k] - b.nodes[0].box.lo[k] > kMaxSurfExtent) return;
     const Collapse collapse(b.nodes);
     struct Item { int32_t binary; size_t wide; int level; };
     std::vector<Item> queue = {{0, 0, 1}};

@@ -119,9 +119,9 @@ __device__ __forceinline__ void walk_begin(const DevScene& sc, v3 s, v3 d, WalkW
     w->leaf[lane] = kNoLeaf;
     l->key = kNoKey;
     float fdx = (float)d.x, fdy = (float)d.y, fdz = (float)d.z;
-    if (fabsf(fdx) < 1e-30f) fdx = copysignf(1e-30f, fdx);
-    if (fabsf(fdy) < 1e-30f) fdy = copysignf(1e-30f, fdy);
-    if (fabsf(fdz) < 1e-30f) fdz = copysignf(1e-30f, fdz);
+    if (fabsf(fdx) < kMinDirection) fdx = copysignf(kMinDirection, fdx);
+    if (fabsf(fdy) < kMinDirection) fdy = copysignf(kMinDirection, fdy);
+    if (fabsf(fdz) < kMinDirection) fdz = copysignf(kMinDirection, fdz);
     l->ix = 1.0f/fdx; l->iy = 1.0f/fdy; l->iz = 1.0f/fdz;
     l->ox = (float)s.x; l->oy = (float)s.y; l->oz = (float)s.z;
     l->eps = sc.bvh_eps + 4e-7f*(fabsf(l->ox) + fabsf(l->oy) + fabsf(l->oz));

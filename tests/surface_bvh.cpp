@@ -25,7 +25,7 @@ void candidates(const SurfBvhHost& b, const double* s, const double* d, float ep
     for (int a = 0; a < 3; a++) {
         o[a] = (float)s[a];
         float f = (float)d[a];
-        if (std::fabs(f) < 1e-30f) f = std::copysign(1e-30f, f);
+        if (std::fabs(f) < mlgpu::kMinDirection) f = std::copysign(mlgpu::kMinDirection, f);
         iv[a] = 1.0f/f;
     }
     w = eps + 4e-7f*(std::fabs(o[0]) + std::fabs(o[1]) + std::fabs(o[2]));
@@ -43,7 +43,7 @@ void candidates(const SurfBvhHost& b, const double* s, const double* d, float ep
                 const float W = w*std::fabs(iv[a]);
                 const float ql = 32768.0f + (float)((n.qlo[a][k >> 2] >> (8*(k & 3))) & 0xff);
                 const float qh = 32768.0f + (float)((n.qhi[a][k >> 2] >> (8*(k & 3))) & 0xff);
-                const bool back = d[a] < 0.0;
+                const bool back = iv[a] < 0.0f;   // as the kernel: -0 is a negative direction
                 const float x = std::fma(back ? qh : ql, S, L - W), y = std::fma(back ? ql : qh, S, L + W);
                 tmin = std::fmax(tmin, x);
                 tmax = std::fmin(tmax, y);

@@ -51,3 +51,24 @@ def check(oracle, name, ph, pool, order=0):
     got = {k: v.cpu().numpy() for k, v in out.items()}
     assert mismatches(ref, got) == {}
     scene.close()
+
+
+@pytest.mark.parametrize("radius", [1e2, 3e6, 1e9, 1e17])
+@pytest.mark.parametrize("n", [2000, 70_003])
+def test_wide_sceneries_and_rays_along_the_axes(oracle, radius, n):
+    """Steps of a node's bounds over a direction component of zero stay finite;
+    beyond the largest extent the level kernels take over."""
+    from merlict_development_kit_b200 import engine
+    from test_surface_bvh import along_the_axes, wide_scene
+    flat = wide_scene(radius)
+    ph = along_the_axes(n, 4)
+    status, ref, _ = oracle.propagate(flat, ph, 3, seed=5)
+    assert status == 0
+    scene = engine.Scene(flat)
+    out = scene.propagate(engine.photons_to_device(ph), engine.PropagationConfig(3),
+                          engine.Philox(5), outputs=("sensor", "final_leaf", "info", "time",
+                                                     "final_position", "final_direction"))
+    got = {k: v.cpu().numpy() for k, v in out.items()}
+    assert (ref["final_leaf"] >= 0).sum() > 0.5*n
+    assert mismatches(ref, got) == {}
+    scene.close()

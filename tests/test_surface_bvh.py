@@ -149,3 +149,45 @@ def test_degenerate_surfaces_keep_their_spheres(checker):
             C.c_void_p(leaf.ctypes.data), C.byref(visits)) == 0
         checked += 1
     assert checked >= 1
+
+
+def wide_scene(radius):
+    """A ground disc of `radius` under a few small surfaces."""
+    from merlict_development_kit_b200 import scenery as S
+    sc = S.Scenery()
+    sc.root.add(S.Disc("ground", (0.0, 0.0, -2.0), S.ROT3_UNITY)).set_radius(radius)
+    for i in range(20):
+        d = sc.root.add(S.Disc(f"d{i}", (3.0*i, -2.0*i, 0.1*i), S.Rot3(0.02*i, -0.01*i, 0.0)))
+        d.set_radius(0.5)
+        s = sc.root.add(S.Sphere(f"s{i}", (-3.0*i - 1.5, 2.0*i, 5.0), S.ROT3_UNITY))
+        s.set_radius(0.7)
+    sc.init()
+    return sc.flatten()
+
+
+def along_the_axes(n, seed):
+    """Rays with one or two components that are exactly zero."""
+    rng = np.random.default_rng(seed)
+    d = np.zeros((n, 3))
+    d[:, 2] = -1.0
+    d[1::4] = [0.0, 0.6, -0.8]
+    d[2::4] = [-1.0, -0.0, 0.0]
+    d[3::4, 0] = 1e-25
+    sup = rng.uniform(-60.0, 60.0, size=(n, 3))
+    sup[:, 2] = rng.uniform(0.0, 30.0, n)
+    return P.make_batch(sup, d, np.full(n, 433e-9))
+
+
+@pytest.mark.parametrize("radius", [1e2, 1e6, 2e6, 3e6, 1e7, 1e9, 1e13])
+def test_wide_sceneries_and_rays_along_the_axes(checker, oracle, radius):
+    flat = wide_scene(radius)
+    assert consistent(checker, flat)[2] >= 1
+    assert reaches_every_hit(checker, oracle, flat, along_the_axes(2000, 3)) > 1000
+
+
+def test_no_surface_tree_beyond_the_largest_extent(checker):
+    flat = wide_scene(1e17)
+    s = flat.as_struct()
+    info = (C.c_int64 * 3)()
+    assert checker.surface_bvh_invariants(C.byref(s), info) == 0
+    assert list(info) == [0, 0, 0]
