@@ -727,13 +727,7 @@ int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, bool whole, cuda
     w.fn_smem_bytes = table_smem_bytes(scene);
     const uint64_t n = a->num_photons;
     if (!whole && n >= (1ull << 31)) return MLGPU_OK;
-    Profiler::Chain ch;
-    const bool timed = scene->prof.on && scene->prof.take(2, ch.ev);
-    if (timed) cudaEventRecord(ch.ev[0], stream);
-    cudaError_t e;
-    if (whole) {
-        e = launch_wave_finish(*a, w, none, kFinishBatchMode, (uint32_t)n, stream);
-    } else {
+    if (!whole) {
         const int rc = wave_host_counters(scene);
         if (rc) return rc;
         MLGPU_CUDA(scene->order.reserve(256 + kWaveCounterBytes + 4*n));
@@ -741,23 +735,28 @@ int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, bool whole, cuda
         w.counters = reinterpret_cast<WaveCounters*>(b);
         w.first = reinterpret_cast<uint32_t*>(b + kWaveCounterBytes);
         MLGPU_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(WaveCounters), stream));
+    }
+    ProfileMark mark;
+    profile_mark_begin(scene, stream, &mark);
+    cudaError_t e;
+    int traced = 1;
+    if (whole) {
+        e = launch_wave_finish(*a, w, none, kFinishBatchMode, (uint32_t)n, stream);
+    } else {
         e = launch_wave_first(*a, w, stream);
         if (e == cudaSuccess && want >= kFinishRays) {
             TraceArgs l = *a;
             l.order = w.first;
             e = launch_wave_finish(l, w, none, kFinishListMode, kFinishRays, stream);
-            scene->launches++;
+            traced++;
         }
-        if (e == cudaSuccess)
-            e = launch_wave_counters_to_host(w.counters, scene->wave_host_dev, stream);
-        scene->launches++;
     }
     if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
-    scene->launches++;
-    if (timed) {
-        cudaEventRecord(ch.ev[1], stream);
-        ch.n = 2; ch.cls[0] = MLGPU_KERNEL_PLAIN; ch.launches[0] = 1;
-        scene->prof.add(ch);
+    profile_mark_end(scene, stream, &mark, MLGPU_KERNEL_PLAIN, traced);
+    if (!whole) {
+        e = launch_wave_counters_to_host(w.counters, scene->wave_host_dev, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "wavefront counters");
+        scene->launches++;
     }
     *done = whole;
     if (!whole) {
@@ -913,10 +912,12 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
         if (left == 0 && h.next_input >= a.num_photons) break;
         if (finish && left <= kFinishRays && h.next_input >= a.num_photons) {
             // the last rays, in one launch
+            ProfileMark mark;
+            profile_mark_begin(scene, stream, &mark);
             const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], kFinishPoolMode, left,
                                                      stream);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
-            scene->launches++;
+            profile_mark_end(scene, stream, &mark, MLGPU_KERNEL_PLAIN, 1);
             for (int c = 0; feed && c < feed->pieces; c++) {
                 if (downloaded[c]) continue;
                 const int r = feed->download(c);

@@ -72,3 +72,33 @@ def test_wide_sceneries_and_rays_along_the_axes(oracle, radius, n):
     assert (ref["final_leaf"] >= 0).sum() > 0.5*n
     assert mismatches(ref, got) == {}
     scene.close()
+
+
+@pytest.mark.parametrize("n,sparse,plain", [(20_011, False, 1),    # one launch for the batch
+                                            (100_003, True, 2),    # first look, the listed ones
+                                            (300_001, False, 3)])  # and the pool's last rays
+def test_every_kernel_of_a_call_is_in_a_class(n, sparse, plain):
+    """Launches counted are launches timed, but for the copies of the counters
+    to the host, one before each of the host's looks."""
+    from merlict_development_kit_b200 import engine
+    flat, _, _, meta = load_golden("light_field_small")
+    scene = engine.Scene(flat)
+    ph = engine.photons_to_device(batch("sparse" if sparse else "light_field_small", n))
+    config = engine.PropagationConfig(meta["max_interactions"])
+    scene.propagate(ph, config)
+    scene.set_profiling(True)
+    before = scene.kernel_launches(), scene.wavefront_stats()["iterations"]
+    scene.propagate(ph, config)
+    launches = scene.kernel_launches() - before[0]
+    iterations = scene.wavefront_stats()["iterations"] - before[1]
+    times = scene.kernel_times()
+    scene.set_profiling(False)
+    timed = {k: count for k, (ms, count) in times.items() if count}
+    assert timed["plain"] == plain and times["plain"][0] > 0.0
+    if plain < 3:
+        assert set(timed) == {"plain"} and launches == plain + (plain > 1)
+    else:
+        assert timed["walk"] == timed["resolve"] == iterations
+        # looks: behind the first look, the first iteration, every second one
+        assert launches == sum(timed.values()) + 2 + iterations//2
+    scene.close()
