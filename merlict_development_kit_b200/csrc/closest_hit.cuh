@@ -240,10 +240,11 @@ __device__ __forceinline__ double leaf_distance(const DevScene& sc, int32_t leaf
             return -1.0;
         Isec h;   // only the distance is used; the rest is not computed
         const v3 ls = position_inverse(T, ti, s), ld = orientation_inverse(T, d);
-        if (kClass == kLeafCap) intersect_cap(sc, leaf, prim, pr, r2, ls, ld, &h);
-        else if (kClass == kLeafPlane) intersect_plane(sc, leaf, prim, pr, ls, ld, &h);
-        else if (kClass == kLeafQuadric) intersect_quadric(leaf, prim, pr, ls, ld, &h);
-        else intersect_leaf(sc, leaf, prim, pr, r2, ls, ld, &h);
+        switch (kClass >= 0 ? kClass : leaf_class(prim)) {
+        case kLeafCap: intersect_leaf<kLeafCap>(sc, leaf, prim, pr, r2, ls, ld, &h); break;
+        case kLeafPlane: intersect_leaf<kLeafPlane>(sc, leaf, prim, pr, r2, ls, ld, &h); break;
+        default: intersect_leaf<kLeafQuadric>(sc, leaf, prim, pr, r2, ls, ld, &h); break;
+        }
         return h.leaf >= 0 ? h.dist : -1.0;
     }
     const fp32::Hit32 h = fp32::intersect32<false>(sc, leaf, fp32::dmk(s.x, s.y, s.z),

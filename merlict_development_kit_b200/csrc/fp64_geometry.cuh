@@ -233,15 +233,20 @@ __device__ __forceinline__ double tri_sign(v3 p1, double p2x, double p2y, double
 }
 
 // calculate_intersection_with of the leaf primitives
-// (merlict/scenery/primitive), ray given in the leaf's frame, in three
-// classes of arithmetic (leaf_class).
-__device__ __forceinline__ void intersect_cap(const DevScene& sc, int32_t leaf, int32_t prim,
-                                              const double* pr, double r2, v3 s, v3 d, Isec* out) {
+// (merlict/scenery/primitive), ray given in the leaf's frame.  kClass: the
+// class of arithmetic (leaf_class) that the leaf is known to be of, or -1
+// for one switch over all: the plain tracer takes 1.57 ms per 1e6 photons of
+// the reflector camera so, and 1.73 with a switch over the classes first,
+// which the closest-hit walk's lens search is 3 % faster with.
+template <int kClass>
+__device__ __forceinline__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
+                                               const double* pr, double r2, v3 s, v3 d, Isec* out) {
     out->leaf = -1;
     switch (prim) {
     case MLGPU_PRIM_SPHERE_CAP_HEX:
     case MLGPU_PRIM_SPHERE_CAP_CYL:
     case MLGPU_PRIM_SPHERE_CAP_RECT: {
+        if (kClass >= 0 && kClass != kLeafCap) break;
         const double R = pr[0];
         const double dd = dot(d, d), ss = dot(s, s), sd = dot(s, d);
         const double Rdz = R*d.z, Rsz = R*s.z;
@@ -253,6 +258,7 @@ __device__ __forceinline__ void intersect_cap(const DevScene& sc, int32_t leaf, 
         break;
     }
     case MLGPU_PRIM_ELLIPTIC_CAP_HEX: {
+        if (kClass >= 0 && kClass != kLeafCap) break;
         const double C = pr[2], iAA = pr[3], iBB = pr[4], iCC = pr[5];
         const double a = (d.x*d.x)*iAA + (d.y*d.y)*iBB + (d.z*d.z)*iCC;
         const double b = 2.0*((s.x*d.x)*iAA + (s.y*d.y)*iBB + d.z*(s.z - C)*iCC);
@@ -262,21 +268,13 @@ __device__ __forceinline__ void intersect_cap(const DevScene& sc, int32_t leaf, 
             add_causal(sc, leaf, prim, pr, r2, plus, minus, s, d, out);
         break;
     }
-    default:
-        break;
-    }
-}
-
-__device__ __forceinline__ void intersect_plane(const DevScene& sc, int32_t leaf, int32_t prim,
-                                                const double* pr, v3 s, v3 d, Isec* out) {
-    out->leaf = -1;
-    switch (prim) {
     case MLGPU_PRIM_DISC:
     case MLGPU_PRIM_HEX_PLANE:
     case MLGPU_PRIM_PLANE:
     case MLGPU_PRIM_ANNULUS:
     case MLGPU_PRIM_PLANE_DUAL_SPHERE:
     case MLGPU_PRIM_TRIANGLE: {
+        if (kClass >= 0 && kClass != kLeafPlane) break;
         // XyPlaneRayIntersectionEquation.cpp:6-40
         const bool parallel = d.z == 0. && (d.x != 0. || d.y != 0.);
         if (parallel) break;
@@ -309,16 +307,8 @@ __device__ __forceinline__ void intersect_plane(const DevScene& sc, int32_t leaf
         if (inside && differs(s, p)) set_isec(out, leaf, p, mk(0.0, 0.0, 1.0), v, d);
         break;
     }
-    default:
-        break;
-    }
-}
-
-__device__ __forceinline__ void intersect_quadric(int32_t leaf, int32_t prim, const double* pr,
-                                                  v3 s, v3 d, Isec* out) {
-    out->leaf = -1;
-    switch (prim) {
     case MLGPU_PRIM_CYLINDER: {
+        if (kClass >= 0 && kClass != kLeafQuadric) break;
         // ZaxisCylinderRayIntersectionEquation.cpp:6-86, Cylinder.cpp:121-150
         const double radius = pr[0], length = pr[1];
         const double dx2 = d.x*d.x, dy2 = d.y*d.y;
@@ -343,6 +333,7 @@ __device__ __forceinline__ void intersect_quadric(int32_t leaf, int32_t prim, co
         break;
     }
     case MLGPU_PRIM_SPHERE: {
+        if (kClass >= 0 && kClass != kLeafQuadric) break;
         // Sphere.cpp:50-104
         const double radius = pr[0];
         const double sd = dot(s, d), dd = dot(d, d), ss = dot(s, s);
@@ -359,15 +350,6 @@ __device__ __forceinline__ void intersect_quadric(int32_t leaf, int32_t prim, co
     }
     default:
         break;
-    }
-}
-
-__device__ __forceinline__ void intersect_leaf(const DevScene& sc, int32_t leaf, int32_t prim,
-                                               const double* pr, double r2, v3 s, v3 d, Isec* out) {
-    switch (leaf_class(prim)) {
-    case kLeafCap: intersect_cap(sc, leaf, prim, pr, r2, s, d, out); break;
-    case kLeafPlane: intersect_plane(sc, leaf, prim, pr, s, d, out); break;
-    default: intersect_quadric(leaf, prim, pr, s, d, out); break;
     }
 }
 
@@ -407,7 +389,7 @@ __device__ __forceinline__ void test_candidate(const DevScene& sc, int32_t leaf,
     for (int k = 0; k < MLGPU_LEAF_PARAMS; k++) pr[k] = __ldg(&L->params[k]);
     const int32_t prim = __ldg(&L->primitive);
     Isec cand;
-    intersect_leaf(sc, leaf, prim, pr, r2, position_inverse(T, ti, s),
+    intersect_leaf<-1>(sc, leaf, prim, pr, r2, position_inverse(T, ti, s),
                    orientation_inverse(T, d), &cand);
     if (cand.leaf >= 0 && (!*have || cand.dist < best->dist ||
                            (cand.dist == best->dist && cand.leaf < best->leaf))) {

@@ -333,7 +333,7 @@ wave_isect_kernel(const TraceArgs a, const WaveBuffers w, const RayPool cur) {
             // conservative single-precision version of it
             if (sphere_cull(make_double4(T[3], T[7], T[11], r2), s, d, dot(s, d))) {
                 Isec h;
-                intersect_leaf(sc, (int32_t)q.y, prim, pr, r2, position_inverse(T, ti, s),
+                intersect_leaf<-1>(sc, (int32_t)q.y, prim, pr, r2, position_inverse(T, ti, s),
                                orientation_inverse(T, d), &h);
                 if (h.leaf >= 0) dist = h.dist;
             }
