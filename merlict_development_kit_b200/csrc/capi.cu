@@ -773,8 +773,10 @@ int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, bool whole, cuda
     return MLGPU_OK;
 }
 
+// *left: whether kernels of the call may still run when it returns.
 int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
-                  cudaStream_t stream, const FeedPlan* feed = nullptr) {
+                  cudaStream_t stream, bool* left, const FeedPlan* feed = nullptr) {
+    *left = true;
     const int form = st->tracer;
     const int walk = wave_walk(scene, st);
     // the FP32 forms' double-precision parts are contracted as the compiler
@@ -795,6 +797,7 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
     } else if (look) {
         bool done = false;
         const int r = first_look(scene, &a, want, whole, stream, &done);
+        if (done) *left = whole;
         if (r || done) return r;
     } else if (walk != MLGPU_WALK_STACK || st->photon_order == MLGPU_ORDER_COHERENT) {
         const int ro = tracing_order(scene, &a, st, stream, true);
@@ -908,13 +911,16 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
             }
         }
         more = h.next_input < a.num_photons;
-        const uint32_t left = h.active + h.inside;
-        if (left == 0 && h.next_input >= a.num_photons) break;
-        if (finish && left <= kFinishRays && h.next_input >= a.num_photons) {
+        const uint32_t rays = h.active + h.inside;
+        if (rays == 0 && h.next_input >= a.num_photons) {
+            *left = false;
+            break;
+        }
+        if (finish && rays <= kFinishRays && h.next_input >= a.num_photons) {
             // the last rays, in one launch
             ProfileMark mark;
             profile_mark_begin(scene, stream, &mark);
-            const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], kFinishPoolMode, left,
+            const cudaError_t e = launch_wave_finish(a, w, pools[iteration & 1], kFinishPoolMode, rays,
                                                      stream);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront kernels");
             profile_mark_end(scene, stream, &mark, MLGPU_KERNEL_PLAIN, 1);
@@ -935,12 +941,13 @@ int run_wavefront(mlgpu_scene* scene, TraceArgs a, const mlgpu_settings* st,
 }
 
 int launch_tracer(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, bool* left) {
     cudaError_t e;
+    *left = true;
     switch (st->tracer) {
     case MLGPU_TRACER_FP64:
     case MLGPU_TRACER_FP32:
-    case MLGPU_TRACER_FP32_PURE: return run_wavefront(scene, a, st, stream);
+    case MLGPU_TRACER_FP32_PURE: return run_wavefront(scene, a, st, stream, left);
     case MLGPU_TRACER_FP64_QUEUE: {
         TraceArgs q = a;
         MLGPU_CUDA(scene->in_flight.wait(stream));
@@ -986,8 +993,9 @@ int launch_tracer(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* 
 // One propagation, its last kernels left in flight.
 int launch(mlgpu_scene* scene, const TraceArgs& a, const mlgpu_settings* st,
            cudaStream_t stream) {
-    const int rc = launch_tracer(scene, a, st, stream);
-    const cudaError_t e = scene->in_flight.mark(stream);
+    bool left = true;
+    const int rc = launch_tracer(scene, a, st, stream, &left);
+    const cudaError_t e = left ? scene->in_flight.mark(stream) : cudaSuccess;
     if (rc == MLGPU_OK && e != cudaSuccess) return cuda_fail(e, "event behind a propagation");
     return rc;
 }
@@ -1664,7 +1672,8 @@ int propagate_host(mlgpu_scene* scene, const mlgpu_photons* photons, uint64_t n,
         dres.final_direction = static_cast<double*>(dev_plane[9]);
         dres.history = static_cast<mlgpu_history_entry*>(dev_plane[10]);
         const TraceArgs a = make_args(scene, &dph, n, settings, &drng, &dres);
-        st = run_wavefront(scene, a, settings, trace, &plan);
+        bool left = true;   // the call waits for its streams at its end
+        st = run_wavefront(scene, a, settings, trace, &left, &plan);
         if (st) return drain(st);
     }
     for (int c = 0; !fed && c < pieces; c++) {

@@ -210,27 +210,26 @@ class Scene:
         }
         wanted = set(outputs) | {"sensor"}
         made = history
-        used = [photons[k] for k in PLANES]
         for k, (shape, dt) in spec.items():
             if k in wanted:
                 if k not in out or out[k].shape[0] < n:
                     out[k] = torch.empty(shape, dtype=dt, device=dev)
                     made = True
                 setattr(res, k, out[k].data_ptr())
-                used.append(out[k])
         if history:
             m = config.max_num_interactions_per_photon + 1
             out["history"] = torch.empty((n, m, abi.HISTORY_DTYPE.itemsize), dtype=torch.uint8, device=dev)
             res.history = out["history"].data_ptr()
-            used.append(out["history"])
+            wanted.add("history")
         st = _settings(config, start_node, tracer, traversal, tuning)
         r, keep = rng._struct(n)
-        if made or (keep is not None and keep is not rng.uniforms):
+        if stream is not None and (made or (keep is not None and keep is not rng.uniforms)):
             _behind_current(stream)
         sh = _stream_handle(stream)
         rc = lib().mlgpu_propagate(self._h, C.byref(ph), n, C.byref(st), C.byref(r),
                                    C.byref(res), C.c_void_p(sh))
-        _in_use(stream, keep, *used)
+        if stream is not None:
+            _in_use(stream, keep, *(photons[k] for k in PLANES), *(out[k] for k in wanted if k in out))
         check(rc)
         rng.advance(n)
         if sync:

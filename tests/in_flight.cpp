@@ -23,7 +23,8 @@ void merge(Past* to, const Past& from) {
     for (const auto& p : from) (*to)[p.first] = std::max((*to)[p.first], p.second);
 }
 
-cudaStream_t handle(int k) { return reinterpret_cast<cudaStream_t>((intptr_t)(16 + k)); }
+// stream 0 is the default stream, which is never another
+cudaStream_t handle(int k) { return reinterpret_cast<cudaStream_t>((intptr_t)(k ? 16 + k : 0)); }
 
 void work(cudaStream_t s) { streams[s][s]++; }
 
@@ -74,7 +75,7 @@ int64_t in_flight_violations(int num, int steps, uint32_t seed) {
             f.wait(s);
             if (!after(s, marked)) bad++;
         }
-        if (rng() % 16 == 0) {                      // the handle of another stream now
+        if (s != nullptr && rng() % 16 == 0) {      // the handle of another stream now
             streams[s] = Past();
             ids[s] = next_id++;
             if (rng() % 2) { f.wait(s); if (!after(s, marked)) bad++; }
@@ -108,6 +109,8 @@ int64_t in_flight_capture() {
     mlgpu::InFlight f;
     work(handle(0));
     f.mark(handle(0));
+    work(handle(2));
+    f.mark(handle(2));
     captures[handle(1)] = true;
     const int64_t before = waits, had = live_events;
     f.wait(handle(1));

@@ -40,7 +40,7 @@ def test_two_batches_on_two_streams(telescope, tracer, n):
                for k in range(4)]
     kw = dict(outputs=OUT, tracer=tracer)
     one_by_one = [scene.propagate(b, config, engine.Philox(k), **kw) for k, b in enumerate(batches)]
-    streams = [torch.cuda.Stream() for _ in range(3)]
+    streams = [torch.cuda.default_stream(), torch.cuda.Stream(), torch.cuda.Stream()]
     torch.cuda.synchronize()
     for _ in range(3):
         got = [scene.propagate(b, config, engine.Philox(k), stream=streams[k % 3], sync=False, **kw)
