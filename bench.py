@@ -42,9 +42,13 @@ BYTES_PER_PHOTON = {"fp64": 88, "fp64_plain": 88, "fp32": 52}
 # Fresnel steps, time-of-flight segments, table look-ups)
 FLOP_WEIGHTS = {"nodes": 26, "leaves": 48, "caps": 29, "cap_bounds": 85, "planes": 36,
                 "others": 29, "reflections": 91, "fresnels": 110, "segments": 3, "funcs": 4}
-# the kernel class that does each counted operation (the closest-hit walk
-# intersects the leaves it finds)
-FLOP_STAGE = {"nodes": "walk", "leaves": "walk", "caps": "walk", "cap_bounds": "walk",
+# The kernel class that does each counted operation.  merlict's search tests
+# the spheres of 412.7 nodes per photon and intersects 21.0 leaves; the
+# closest-hit walk visits 27.8 nodes of its own tree in single precision and
+# takes WALK_LEAVES leaves through merlict's sphere test and intersection, so
+# it is credited with those.
+WALK_LEAVES = 13.0
+FLOP_STAGE = {"leaves": "walk", "caps": "walk", "cap_bounds": "walk",
               "planes": "walk", "others": "walk", "reflections": "resolve",
               "fresnels": "resolve", "segments": "resolve", "funcs": "resolve"}
 FP64_PEAK_TFLOPS_NOMINAL = 37.0   # B200 vector FP64 with FMAs, nominal
@@ -421,8 +425,11 @@ def run_ours(args, world, rank, local):
     counts = flop_counts()
     per = counts["per_photon"] if counts else {}
     stage_flops = {}
-    for k, w in FLOP_WEIGHTS.items():
-        stage_flops[FLOP_STAGE[k]] = stage_flops.get(FLOP_STAGE[k], 0.0) + w * per.get(k, 0.0)
+    for k, stage_of in FLOP_STAGE.items():
+        done = WALK_LEAVES / per["leaves"] if per and stage_of == "walk" else 1.0
+        stage_flops[stage_of] = (stage_flops.get(stage_of, 0.0) +
+                                 done * FLOP_WEIGHTS[k] * per.get(k, 0.0))
+    stage_flops["walk"] += FLOP_WEIGHTS["nodes"] * WALK_LEAVES   # the leaves' sphere tests
     total_stage_ms = sum(ms for ms, _ in stage.values())
     kernels = {}
     for name, (ms, nl) in stage.items():
@@ -435,9 +442,9 @@ def run_ours(args, world, rank, local):
                          "tflops": f / (ms * 1e-3) / 1e12 if ms > 0 else None}
     dominant = max(kernels, key=lambda k: kernels[k]["ms_per_step"])
     dk = kernels[dominant]
-    # the dominant stage against the vector pipe that bounds it: the
-    # reference's operation counts for that stage, per photon, times the
-    # photons of a step, over the stage's device time per step
+    # the dominant stage against the vector pipe: the operations it does of
+    # those that the reference counts, per photon, times the photons of a
+    # step, over the stage's device time per step
     achieved = dk["flops_per_photon"] * n / (dk["ms_per_step"] * 1e-3) / 1e12
     # the denominator, measured on this GPU: separate FP64 adds and
     # multiplies (the reference's operations, which the bit-exact tracer may
@@ -459,10 +466,15 @@ def run_ours(args, world, rank, local):
                 "frac_of_fma_peak": achieved / (rate_fma.value / 1e12),
                 "peak_fp64_nominal": FP64_PEAK_TFLOPS_NOMINAL,
                 "flops_per_photon": dk["flops_per_photon"]}
+    # the whole call: by the operations done, and beside it by all that the
+    # reference's own traversal counts, most of whose search is left out here
     flops = sum(stage_flops.values())
-    whole = flops * n / (kernel_ms * 1e-3) / 1e12
-    compute = {"bound": roofline["bound"], "flops_per_photon": flops, "achieved": whole,
-               "peak": peak, "unit": "TFLOP/s", "frac": whole / peak,
+    reference_flops = sum(w * per.get(k, 0.0) for k, w in FLOP_WEIGHTS.items())
+    rate = n / (kernel_ms * 1e-3) / 1e12
+    compute = {"bound": roofline["bound"], "flops_per_photon": flops, "achieved": flops * rate,
+               "peak": peak, "unit": "TFLOP/s", "frac": flops * rate / peak,
+               "reference_flops_per_photon": reference_flops,
+               "reference_flops_frac": reference_flops * rate / peak,
                "scope": "whole propagate call"}
     achieved_gbs = bpp * n / (kernel_ms * 1e-3) / 1e9
     hbm = {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
