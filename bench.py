@@ -53,7 +53,8 @@ FLOP_STAGE = {"leaves": "walk", "caps": "walk", "cap_bounds": "walk",
               "fresnels": "resolve", "segments": "resolve", "funcs": "resolve"}
 FP64_PEAK_TFLOPS_NOMINAL = 37.0   # B200 vector FP64 with FMAs, nominal
 # DRAM bytes per photon of each kernel class on the light-field telescope,
-# from an ncu capture of one propagation of 4e6 photons (dram__bytes_read.sum
+# from an ncu capture of one propagation of 4e6 photons in the input order
+# (dram__bytes_read.sum
 # + dram__bytes_write.sum summed over the class's launches, divided by the
 # photons; profiles/wavefront_fp64_light_field_telescope.md): walk = the
 # closest-hit walks; resolve = the interactions; plain = the first look at

@@ -232,7 +232,8 @@ typedef struct mlgpu_settings {
     int32_t block_size;     /* 0 = default                                    */
     int32_t traversal;      /* MLGPU_TRAVERSAL_*                              */
     uint32_t pool_size;     /* ray slots of the wavefront pool (2^23; 2^21 for
-                               the LEVELS walk and the host-buffer calls)      */
+                               the LEVELS walk and for a fed host call, see
+                               mlgpu_propagate_host)                           */
     int32_t check_period;   /* iterations between host checks of the pool (4) */
     int32_t use_graph;      /* 1: each check period is one CUDA-graph launch  */
     int32_t grid_blocks;    /* blocks of the grid-stride kernels (8 per SM)   */
@@ -261,10 +262,11 @@ enum { MLGPU_WALK_DEFAULT = 0, MLGPU_WALK_LEVELS = 1, MLGPU_WALK_STACK = 2 };
 /* photon_order: COHERENT sorts the batch by a 4-D cell key of support and
  * direction before tracing, so that neighbouring ray slots follow nearly
  * the same path (results are the same in any order).  DEFAULT is INPUT for
- * the STACK walk on device buffers, which gains no more from the order than
- * the sort costs; for the LEVELS walk, the work-queue tracer and the
- * host-buffer calls it is COHERENT for batches of at least 65,536 photons
- * and INPUT below.                                                         */
+ * the STACK walk, which gains little from the order and loses on small and
+ * sparse batches; for the LEVELS walk, the work-queue tracer and a fed host
+ * call (page-locked buffers and at least a ray pool of photons, see
+ * mlgpu_propagate_host) it is COHERENT for batches of at least 65,536
+ * photons and INPUT below.  Other host calls are as calls on device buffers. */
 enum { MLGPU_ORDER_DEFAULT = 0, MLGPU_ORDER_INPUT = 1, MLGPU_ORDER_COHERENT = 2 };
 
 typedef struct mlgpu_scene mlgpu_scene;
@@ -551,13 +553,17 @@ int mlgpu_signal_chain(
 /* ---- tuning ------------------------------------------------------------ *
  * No counterpart in the reference (merlict has no device parameters).
  * Picks the wavefront knobs of `base` (pool_size, check_period, use_graph,
- * grid_blocks, staged_levels, photon_order) for this scene by timing
+ * grid_blocks, staged_levels, photon_order, walk) for this scene by timing
  * mlgpu_propagate on a
  * sample of photons (device pointers, as for mlgpu_propagate): coordinate
  * descent from the defaults, each candidate timed with CUDA events on
- * `cuda_stream` (best of two runs after one untimed run).  Writes the
- * fastest settings to `best` (the other fields copied from `base`) and its
- * time in milliseconds to `best_ms` (may be NULL).  Results of the sample
+ * `cuda_stream` (best of four runs after one untimed run).  A knob leaves
+ * its value for one that is 2 % faster or more.  Pools from 2^19 to 2^23 ray
+ * slots are tried, none of more than twice the sample and, for the STACK
+ * walk, none below 2^21: it gains with every larger pool, which a sample that
+ * does not fill them cannot show.  Writes the settings to `best` (the other
+ * fields copied from `base`) and their time on the sample in milliseconds to
+ * `best_ms` (may be NULL).  Results of the sample
  * runs are discarded; the tracer form is `base->tracer` (a wavefront
  * form).  The knobs never change what a propagation computes.            */
 int mlgpu_scene_autotune(

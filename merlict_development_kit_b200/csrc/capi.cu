@@ -542,9 +542,9 @@ TraceArgs make_args(const mlgpu_scene* scene, const mlgpu_photons* ph, uint64_t 
 constexpr uint32_t kWavePool = 1u << 21;
 constexpr uint32_t kWalkPool = 1u << 23;
 
-// How the rays of a call find their hits.  One thread per ray through the
-// surface BVH (STACK) unless the caller asks for the level kernels, by name
-// or by the size of their queues; the pure FP32 form always takes them: its
+// How the rays of a call find their hits: by the warps' walk of the surface
+// BVH (STACK) unless the caller asks for the level kernels, by name or by
+// the size of their queues, or the scene has no such BVH; the pure FP32 form always takes them: its
 // textbook roots can lie further outside a surface than that BVH's boxes.
 int wave_walk(const mlgpu_scene* scene, const mlgpu_settings* st) {
     if (st->tracer == MLGPU_TRACER_FP32_PURE || st->walk == MLGPU_WALK_LEVELS ||
@@ -712,11 +712,12 @@ struct FeedPlan {
 // batch small enough for one launch is traced by it (*done); of a larger
 // one, the photons that miss the scenery end in a first look, and if few are
 // left, one launch ends those as well; else they are a's photons, by index,
-// when this returns.  The input order is the default: sorting 1e7 photons of
-// the light-field telescope takes 1.2 ms and gains the walk as much (18.22
-// against 18.30 ms), smaller and sparser batches lose by it (80,000 photons
-// 467 against 563 us, 25e6 photons of air showers 3.8 against 5.6 ms, 8e6 of
-// the large reflector in FP32 5.3 against 6.2 ms).
+// when this returns.  The input order is the default: sorting gains 1e7
+// photons of the light-field telescope 2 % (16.4 against 16.8 ms), and
+// smaller and sparser batches lose by it: 80,000 telescope photons 541
+// against 485 us, 1e6 photons of one shower 564 against 377 us, 1.85e7 of 200
+// showers 5.4 against 1.85 ms, 8e6 of the large reflector in FP32 5.75
+// against 4.87 ms.
 int first_look(mlgpu_scene* scene, TraceArgs* a, uint32_t want, bool whole, cudaStream_t stream,
                bool* done) {
     WaveBuffers w;

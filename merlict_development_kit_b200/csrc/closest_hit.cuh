@@ -25,12 +25,13 @@
 // nodes and intersect 13.0 leaves.  Propagating 1e7 photons, the searches
 // took 22.5 ms as one kernel per BVH level over queued (ray, node) pairs plus
 // intersection and tie kernels, and take 12.9 ms so, of which 1.6 ms are the
-// walks inside lenses.  On the way: one thread per ray with its own leaf list
+// walks inside lenses (of the build that brought the walk).  On the way: one thread per ray with its own leaf list
 // 18.0 ms (15 of 32 lanes busy), refilled lanes and a shared leaf list 18.9,
 // lists by kind 15.9, the same at 116 registers instead of 80 14.4, 32-byte
-// loads instead of 16-byte ones 13.6, leaves queued in groups 12.9; since
-// then 10.1, with the walks inside lenses in the interaction's kernel, 2^23
-// rays at a time and three-way integer minima for the slab test.
+// loads instead of 16-byte ones 13.6, leaves queued in groups 12.9; now 11.3
+// (10.1 in the coherent order), with the walks inside lenses in the
+// interaction's kernel, 2^23 rays at a time and three-way integer minima for
+// the slab test.
 #ifndef MLGPU_CLOSEST_HIT_CUH_
 #define MLGPU_CLOSEST_HIT_CUH_
 

@@ -1,5 +1,18 @@
-// wave_resolve.cuh -- the per-candidate and per-slot steps of the wavefront
-// tracers, shared by the FP64 and FP32 forms:
+// wave_resolve.cuh -- the kernels of the wavefront tracers, shared by the
+// FP64 and FP32 forms.  With the closest-hit walk (the default):
+//   hit        new photons and the pool's rays: the closest hit of each by
+//              the walk of closest_hit.cuh;
+//   resolve    one thread per ray: the winner's point and normal (FP64: at
+//              the distance the walk found; the single-precision forms solve
+//              the winner again with its point refined), the interaction with
+//              the surface (merlict/PhotonAndFrame.cpp:13-124), the history
+//              entry and the time-of-flight term; survivors are compacted into
+//              the next pool with a warp ballot and one atomic per warp,
+//              finished photons write their results;
+//   first      FP64: ends a large batch's photons that miss the scenery and
+//              lists the others;
+//   finish     FP64: photons from where they are to their ends in one launch.
+// With the level kernels (wavefront_fp64.cu), which propose candidate leaves:
 //   intersect  one thread per (ray, candidate leaf): the distance to the
 //              leaf's hit; the smallest distance of each ray is kept with a
 //              64-bit atomic minimum on its bits (positive doubles order like
@@ -9,12 +22,7 @@
 //              visits first (RayAndFrame.cpp:160-173);
 //   overflow   rays whose walk overflowed a queue get merlict's own walk of
 //              the frame tree;
-//   resolve    one thread per ray: the winner's full intersection, recomputed
-//              by the same code, the interaction with the surface
-//              (merlict/PhotonAndFrame.cpp:13-124), the history entry and the
-//              time-of-flight term; survivors are compacted into the next
-//              pool with a warp ballot and one atomic per warp, finished
-//              photons write their results.
+//   resolve    as above.
 //
 // kIsect selects the intersection arithmetic: FP64 (merlict's, bit-identical
 // when the translation unit is compiled with --fmad=false), or the FP32
@@ -621,9 +629,10 @@ __device__ __forceinline__ void stage_tables(const DevScene& sc, int bytes, doub
 // The first look at a large batch: a photon that misses the root frame's
 // sphere (most of an air shower's) ends here, its void result written where
 // it is read, and the others' indices are listed in w.first for the tracer,
-// so that only they pass through the pool.  Streams the planes once: 25e6
-// photons of air showers, 2 % of which are listed, took 5.6 ms through the
-// pool in coherent order and 3.8 ms in input order.
+// so that only they pass through the pool.  Streams the planes once: 1.85e7
+// photons of air showers, 2 % of which are listed, spend 0.42 ms here (3.7
+// TB/s of planes and results) and 1.85 ms in all; through the pool in the
+// coherent order they take 5.4 ms.
 template <typename In, typename Out>
 __global__ void __launch_bounds__(256, 4)
 wave_first_kernel(const TraceArgs a, const WaveBuffers w) {
@@ -677,8 +686,9 @@ wave_first_kernel(const TraceArgs a, const WaveBuffers w) {
 // that wave_first_kernel listed, unless there are more than kFinishRays.  A warp keeps its photons, one per
 // lane, and alternates between searching their hits and resolving them; no
 // host, no counters and no other kernel come between the interactions of a
-// photon.  For few rays that is what counts: a wavefront iteration is four
-// launches however few rays it advances.  With fewer photons than the grid
+// photon.  For few rays that is what counts: a wavefront iteration is two
+// kernels, each with its ramp and its longest ray, however few rays it
+// advances.  With fewer photons than the grid
 // has lanes each warp takes fewer, since a warp lasts as long as its longest
 // photon.
 template <typename In, typename Out>
@@ -845,9 +855,9 @@ __device__ __forceinline__ void resolve_slot(const TraceArgs& a, const WaveBuffe
 // walk of the lens.  96 registers and a few dozen bytes spilled, five blocks
 // of 128 per SM: the step waits on its gathers and on chains of
 // double-precision arithmetic.  1e7 photons of the light-field telescope take
-// 17.65 ms so, and 17.8, 18.0 and 18.1 ms with six to eight blocks.  As three
-// kernels (lens search, resolve, counters) of their own an iteration ended
-// three times: 18.3 ms.
+// 16.8 ms so, and 16.7, 16.9, 17.1 and 17.3 ms with four, six, seven and eight
+// blocks.  As three kernels (lens search, resolve, counters) of their own an
+// iteration ended three times: 18.3 ms of an earlier build, 17.65 so.
 constexpr int kResolveThreads = 128;
 constexpr int kResolveBlocks = 5;
 
