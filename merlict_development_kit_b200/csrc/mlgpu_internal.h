@@ -137,10 +137,11 @@ inline int leaf_class(int32_t primitive) {
     }
 }
 constexpr int kMaxSurfLevels = 64;      // the walk's stack holds one entry per level
-// The closest-hit walk takes no direction component smaller than this.  Over
-// any distance t the ray moves by 1e-20 t, far inside the box widening (4e-7
-// of the distances), and 2^15 steps of a node's bounds over it stay finite
-// for sceneries of up to kMaxSurfExtent; wider ones get no surface BVH.
+// The walks of quantised boxes take no direction component smaller than
+// this.  Over any distance t the ray moves by 1e-20 t, far inside the box
+// widening (4e-7 of the distances), and 2^15 steps of a node's bounds over it
+// stay finite for sceneries of up to kMaxSurfExtent; wider ones get no
+// surface BVH.
 constexpr float kMinDirection = 1e-20f;
 constexpr double kMaxSurfExtent = 1e16;
 

@@ -148,9 +148,9 @@ __device__ __forceinline__ void prepare_levels(const DevScene& sc, const RayPool
     if (step != kStepBvh) return;
     const float ox = (float)s.x, oy = (float)s.y, oz = (float)s.z;
     float fdx = (float)d.x, fdy = (float)d.y, fdz = (float)d.z;
-    if (fabsf(fdx) < 1e-30f) fdx = copysignf(1e-30f, fdx);
-    if (fabsf(fdy) < 1e-30f) fdy = copysignf(1e-30f, fdy);
-    if (fabsf(fdz) < 1e-30f) fdz = copysignf(1e-30f, fdz);
+    if (fabsf(fdx) < kMinDirection) fdx = copysignf(kMinDirection, fdx);
+    if (fabsf(fdy) < kMinDirection) fdy = copysignf(kMinDirection, fdy);
+    if (fabsf(fdz) < kMinDirection) fdz = copysignf(kMinDirection, fdz);
     p.ray_o[slot] = make_float4(ox, oy, oz, box_inflation(sc, ox, oy, oz));
     p.ray_i[slot] = make_float4(1.0f/fdx, 1.0f/fdy, 1.0f/fdz, 0.0f);
 }

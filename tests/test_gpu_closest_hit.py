@@ -102,3 +102,31 @@ def test_every_kernel_of_a_call_is_in_a_class(n, sparse, plain):
         # looks: behind the first look, the first iteration, every second one
         assert launches == sum(timed.values()) + 2 + iterations//2
     scene.close()
+
+
+@pytest.mark.parametrize("walk", [0, 1])
+@pytest.mark.parametrize("tracer", ["fp64", "fp32"])
+def test_rays_along_the_axes_far_from_the_origin(oracle, walk, tracer):
+    """Boxes and rays more than 3.4e8 m from the scenery's origin, where a
+    distance over the smallest direction component must stay finite as well."""
+    from merlict_development_kit_b200 import engine, scenery as S
+    sc = S.Scenery()
+    at = 2.0**31
+    for i in range(12):
+        pos = (at*(i % 3 - 1), -at*(i % 2), at*(i // 6))
+        sc.root.add(S.Sphere(f"s{i}", pos, S.ROT3_UNITY)).set_radius(1024.0)
+    sc.init()
+    flat = sc.flatten()
+    centre = np.asarray(flat.node_sphere).reshape(-1, 4)[np.asarray(flat.leaf_node), :3]
+    n = 1200
+    rng = np.random.default_rng(2)
+    d = np.eye(3)[np.arange(n) % 3]*rng.choice([-1.0, 1.0], size=(n, 1))
+    off = np.round(rng.uniform(-512.0, 512.0, size=(n, 3)))*(1.0 - np.abs(d))
+    ph = P.make_batch(centre[np.arange(n) % 12] + off - 65536.0*d, d, np.full(n, 433e-9))
+    status, ref, _ = oracle.propagate(flat, ph, 1, seed=5)
+    assert status == 0 and (ref["final_leaf"] >= 0).all()
+    scene = engine.Scene(flat)
+    out = scene.propagate(engine.photons_to_device(ph), engine.PropagationConfig(1), engine.Philox(5),
+                          outputs=("sensor", "final_leaf"), tracer=tracer, tuning={"walk": walk})
+    assert np.array_equal(out["final_leaf"].cpu().numpy(), ref["final_leaf"])
+    scene.close()
