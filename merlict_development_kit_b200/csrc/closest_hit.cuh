@@ -84,15 +84,16 @@ inline size_t closest_hit_smem(int levels) {
 // Blocks of a walk over `rays` rays: as many as stay resident, each warp
 // taking several chunks of 32.
 inline int walk_blocks(uint32_t rays) {
-    const uint32_t need = (rays + kWalkThreads - 1)/kWalkThreads;
-    return (int)(need < 148u*kWalkBlocks ? need : 148u*kWalkBlocks);
+    const uint32_t need = (rays + kWalkThreads - 1)/kWalkThreads, full = device_sms()*kWalkBlocks;
+    return (int)(need < full ? need : full);
 }
 
 // Blocks of a launch that takes at most `rays` rays to their ends: a warp
 // per ray up to a full GPU.
 inline int finish_blocks(uint32_t rays) {
     const uint32_t need = (rays + kWalkThreads/32 - 1)/(kWalkThreads/32);
-    return (int)(need < 148u*kFinishBlocks ? need : 148u*kFinishBlocks);
+    const uint32_t full = device_sms()*kFinishBlocks;
+    return (int)(need < full ? need : full);
 }
 
 // A lane's walk.

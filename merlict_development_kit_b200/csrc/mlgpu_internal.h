@@ -330,8 +330,11 @@ struct WaveBuffers {
     uint32_t* first;         // photons that the first look lists for the tracer
 };
 
+// SMs of the device (wavefront_fp64.cu): the launches below fill them.
+unsigned device_sms();
+
 // Batches, lists and remainders that one launch takes to their ends: a lane
-// each on the full GPU (148 SMs of three blocks).  Measured on the
+// each on a B200 (148 SMs of three blocks).  Measured on the
 // light-field telescope: the wavefront is 30-60 us slower for batches up to
 // this size; remainders of up to 8,000, 28,000, 56,832, 120,000 and 250,000
 // rays make 1e6 photons 2.40, 2.40, 2.39, 2.39 and 2.51 ms.

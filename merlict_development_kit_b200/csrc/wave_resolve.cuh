@@ -863,7 +863,8 @@ constexpr int kResolveBlocks = 5;
 
 inline int resolve_blocks(uint32_t pool) {
     const uint32_t need = (pool + kResolveThreads - 1)/kResolveThreads;
-    return (int)(need < 148u*kResolveBlocks ? need : 148u*kResolveBlocks);
+    const uint32_t full = device_sms()*kResolveBlocks;
+    return (int)(need < full ? need : full);
 }
 
 template <typename Out, int kIsect>

@@ -464,7 +464,8 @@ cudaError_t launch_wave_finish(const TraceArgs& a, const WaveBuffers& w, const R
 
 cudaError_t launch_wave_first(const TraceArgs& a, const WaveBuffers& w, cudaStream_t s) {
     const uint64_t tiles = (a.num_photons + 255)/256;
-    const int blocks = (int)(tiles < 148u*8u ? tiles : 148u*8u);
+    const uint64_t full = device_sms()*8u;
+    const int blocks = (int)(tiles < full ? tiles : full);
     const size_t smem = (size_t)w.fn_smem_bytes;
     if (a.in_dtype == MLGPU_F64 && a.out_dtype == MLGPU_F64)
         wave_first_kernel<double, double><<<blocks, 256, smem, s>>>(a, w);
@@ -477,11 +478,17 @@ cudaError_t launch_wave_first(const TraceArgs& a, const WaveBuffers& w, cudaStre
     return cudaGetLastError();
 }
 
-int wave_persistent_blocks() {
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return 8*sms;
+unsigned device_sms() {
+    // of the first device a call is made on; one process works on one GPU
+    static const unsigned sms = [] {
+        int n = 0, dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? (unsigned)n : 1u;
+    }();
+    return sms;
 }
+
+int wave_persistent_blocks() { return 8*(int)device_sms(); }
 
 }  // namespace mlgpu

@@ -286,7 +286,8 @@ class Scene:
                                          C.c_void_p(ids.data_ptr() if ids is not None else None),
                                          C.byref(r), C.byref(buf), C.byref(total),
                                          C.c_void_p(_stream_handle(stream)))
-        _in_use(stream, b, ids, keep, *out.values())
+        if stream is not None:
+            _in_use(stream, b, ids, keep, *out.values())
         check(rc)
         rng.advance(n)
         t = int(total.value)
@@ -342,7 +343,8 @@ class Scene:
             self._h, C.c_void_p(sensor.data_ptr()), C.c_void_p(tp), n,
             C.c_void_p(counts.data_ptr()), C.c_void_p(hist.data_ptr() if hist is not None else None),
             int(num_time_bins), float(t_min), float(t_max), C.c_void_p(_stream_handle(stream)))
-        _in_use(stream, sensor, time if tp is not None else None, counts, hist)
+        if stream is not None:
+            _in_use(stream, sensor, time if tp is not None else None, counts, hist)
         check(rc)
         return counts, hist
 
