@@ -198,3 +198,32 @@ def test_statistics_on_two_streams(telescope):
         torch.cuda.synchronize()
         assert all(torch.equal(a.view(torch.int32), c[0].view(torch.int32))
                    for a, c in zip(want, calls))
+
+
+def test_a_small_batch_in_a_graph(telescope):
+    """A batch of one launch can be captured; calls before, in and behind the
+    capture give what they give without it."""
+    import torch
+    from merlict_development_kit_b200 import engine
+    scene, depth = telescope
+    config = engine.PropagationConfig(depth)
+    small = engine.photons_to_device(P.downward_disc_source(2003, 3, 5.55, 21.4, 0.5))
+    large = engine.photons_to_device(P.downward_disc_source(100_003, 4, 5.55, 21.4, 0.5))
+    want_small = scene.propagate(small, config, engine.Philox(1), outputs=OUT)
+    want_large = scene.propagate(large, config, engine.Philox(2), outputs=OUT)
+    results = {k: torch.empty_like(v) for k, v in want_small.items()}
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    scene.propagate(large, config, engine.Philox(2), outputs=OUT, stream=other, sync=False)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        scene.propagate(small, config, engine.Philox(1), outputs=OUT, results=results, sync=False)
+    for _ in range(2):
+        for v in results.values():
+            v.zero_()
+        graph.replay()
+        got = scene.propagate(large, config, engine.Philox(2), outputs=OUT, stream=other, sync=False)
+        torch.cuda.synchronize()
+        assert equal(want_small, results)
+        assert equal(want_large, got)
